@@ -305,6 +305,7 @@ static int alloc_mesh(tpm_ctx *c) {
   CK(dmalloc(c->arena, &c->tile_start, sizeof(uint32_t) * (ntiles + 1)));
   c->ncubes = 1ll << (3 * (g.cbits - 2));
   CK(dmalloc(c->arena, &c->cube_start, sizeof(uint32_t) * (c->ncubes + 1)));
+  c->tb.units = c->cube_start;
   c->tb.ncubes4 = c->ncubes;
   CK(dmalloc(c->arena, &c->tb.cube_node, sizeof(uint32_t) * c->ncubes));
   CK(dmalloc(c->arena, &c->tb.start_cube, sizeof(uint32_t) * (c->ncubes + 1)));
@@ -519,6 +520,8 @@ WalkBox tpm::ctx_walk_box(const tpm_ctx *c) {
   tp.rsphere = c->prm.rsphere;
   tp.cell_per_unit = (float)((double)c->g.n / 4294967296.0);
   tp.mass = c->prm.particle_mass;
+  tp.group_max = c->tune_group_max;
+  tp.group_level = c->tune_group_level;
   return walk_box(tp, c->spos, c->tb, c->ftree, c->err);
 }
 
@@ -832,11 +835,10 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
     tp.cell_per_unit = (float)((double)g.n / 4294967296.0);
     tp.mass = c->prm.particle_mass;
     tp.group_max = c->tune_group_max;
+    tp.group_level = c->tune_group_level;
     tree_build(tp, c->skey, c->spos, np, c->tb, c->err, st, &c->launches);
     CK(cudaMemsetAsync(c->tb.counters, 0, sizeof(uint32_t) * 16, st));
-    int glev = c->tune_group_level;
-    int64_t gcubes = 1ll << (3 * (g.cbits - glev));
-    tree_groups(tp, c->skey, np, c->tb, c->cube_start, gcubes, 3 * (g.sub_bits + glev), st, &c->launches);
+    tree_targets(tp, c->skey, np, c->tb, c->cube_start, st, &c->launches);
     CK(stage_check(st, "tree_build"));
     // the walk takes every SM: it starts once the PM chain is done too (the
     // tree_build stage of an overlapped evaluation ends with both chains)
@@ -881,7 +883,7 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
       c->stage_ms[s] = ms;
     }
     // counters: nodes, pp, pc, groups
-    uint32_t hc[12];
+    uint32_t hc[16];
     uint32_t lr[2 * (kAxisBits + 2)];
     CK(cudaMemcpy(hc, c->tb.counters, sizeof(hc), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(lr, c->tb.level_range, sizeof(lr), cudaMemcpyDeviceToHost));
@@ -889,12 +891,13 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
     for (int l = 0; l <= kAxisBits; l++)
       if (lr[2 * l + 1] > nn) nn = lr[2 * l + 1];
     c->counters[0] = (parts & TPM_PART_TREE) ? nn : 0;
-    c->counters[1] = (int64_t)(((uint64_t)hc[3] << 32) | hc[2]);
-    c->counters[2] = (int64_t)(((uint64_t)hc[5] << 32) | hc[4]);
-    c->counters[3] = hc[0];
-    c->counters[4] = (int64_t)(((uint64_t)hc[7] << 32) | hc[6]);
-    c->counters[5] = (int64_t)(((uint64_t)hc[9] << 32) | hc[8]);
-    c->counters[6] = hc[10];
+    auto wide = [&](int w) { return (int64_t)(((uint64_t)hc[w + 1] << 32) | hc[w]); };
+    c->counters[1] = wide(kCntPp);
+    c->counters[2] = wide(kCntPc);
+    c->counters[3] = (int64_t)hc[kCntGroups] + hc[kCntSubs];
+    c->counters[4] = wide(kCntIter);
+    c->counters[5] = wide(kCntVisit);
+    c->counters[6] = hc[kCntMaxTop];
   }
   c->parts_valid = parts & TPM_PART_ALL;
   return 0;

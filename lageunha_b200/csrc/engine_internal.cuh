@@ -89,6 +89,10 @@ struct FftPlan {
 };
 // twiddle tables are written on st
 cudaError_t fft_plan_init(FftPlan &p, int n, cudaStream_t st, DeviceArena *arena = nullptr);
+// the same tables in memory of the caller's (fft_twiddles(n) float2), which
+// fft_plan_free must not be called on
+int64_t fft_twiddles(int n);
+cudaError_t fft_plan_in(FftPlan &p, int n, float2 *tw, cudaStream_t st);
 // plain unnormalised transforms: real [z][y][x] -> spec [z][y][hx] (e^{-i}),
 // spec -> ghosted real (e^{+i}; spec is overwritten)
 void fft_forward(const MeshGeom &g, const FftPlan &p, const float *real, float2 *spec, cudaStream_t st);
@@ -129,8 +133,9 @@ struct WalkBox {
   const uint32_t *spos;
   const uint4 *walkA, *walkB;
   const float4 *mom0, *mom1, *mom2;
-  const uint32_t *groups;
-  const uint32_t *ngroups;  // device word: the box's group count
+  uint32_t *groups;         // the groups the walk takes: start, count pairs
+  const uint32_t *units;    // the non-empty 4-cell cubes of the direct summation
+  uint32_t *counters;       // device words, TreeCounter
   float *ftree;
   uint32_t *err;
   // where each group's walk starts: the 4-cell cubes of the tree's level
@@ -138,7 +143,21 @@ struct WalkBox {
   // kNoNode, and the sorted particle range of every cube
   const uint32_t *cube_node, *start_cube;
   float cpu, mass, inv_ll;
-  int n_cells, start_bits;
+  int n_cells, group_max;
+};
+// Words of TreeBuffers::counters (64-bit ones take two).
+enum TreeCounter : int {
+  kCntGroups = 0,     // groups of the tree walk
+  kCntNextGroup = 1,  // its queue head
+  kCntPp = 2,         // particle-particle interactions (64 bits)
+  kCntPc = 4,         // particle-node interactions (64 bits)
+  kCntIter = 6,       // walk iterations (64 bits)
+  kCntVisit = 8,      // nodes the walk examined (64 bits)
+  kCntMaxTop = 10,    // deepest walk stack
+  kCntUnits = 11,     // cubes of the direct summation
+  kCntFofGroups = 12,
+  kCntNextUnit = 13,  // the direct summation's queue head
+  kCntSubs = 14       // its target sub-groups
 };
 constexpr uint32_t kNoNode = 0xffffffffu;
 struct TreeBuffers {
@@ -159,7 +178,8 @@ struct TreeBuffers {
   int64_t cap_tiles = 0;
   uint32_t *groups = nullptr;       // walk groups: start | (count << 26) packed as 2 words
   int64_t cap_groups = 0;
-  uint32_t *counters = nullptr;     // [8]: ngroups, next group, pp, pc, ...
+  uint32_t *counters = nullptr;     // [16], TreeCounter
+  uint32_t *units = nullptr;        // the context's cube_start buffer (ncubes4 words)
   uint32_t *stack = nullptr;        // per-warp global stacks
   int64_t stack_words = 0;
   WalkBox *walkbox = nullptr;       // device copy of this box's walk record
@@ -179,6 +199,7 @@ struct TreeParams {
   float cell_per_unit;  // n / 2^32
   float mass;
   int group_max = 32;   // targets per warp group (<= 32)
+  int group_level = 2;  // groups live in cubes of 2^level cells
 };
 
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
@@ -186,6 +207,19 @@ void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos,
 void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb,
                  uint32_t *cube_start, int64_t ncubes, int cube_shift, cudaStream_t st,
                  int64_t *launches);
+// Whether a box's short-range force starts with the direct summation over
+// its 4-cell cubes (direct.cu): the groups are cut from those cubes, and a
+// cube's reach stays within half a box of any of its targets.
+inline bool direct_applies(const TreeParams &tp) {
+  return tp.group_level == 2 && (float)tp.n >= 2.f * (4.f + tp.rsphere);
+}
+// What the short-range force iterates over: the units of the direct summation
+// where it applies, else every group of the tree walk.
+void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
+                  cudaStream_t st, int64_t *launches);
+// The non-empty 4-cell cubes into tb.units (their count in tb.counters); the
+// direct summation's counterpart of tree_groups.
+void tree_units(TreeBuffers &tb, cudaStream_t st, int64_t *launches);
 // The short-range law's columns on grids uniform in log r^2, indexed by the
 // float bits of s = r^2 + kLogR2Floor (cells^2). Entry k covers
 // [s_k, s_{k+1}), s_k the float whose top bits are (kLogBase + k) <<
@@ -222,6 +256,11 @@ struct LawTable {
   // zero entry)
   uint32_t cut_bits = 0xffffffffu;
 };
+// Direct summation over the units of every box (boxes: device array; uprefix:
+// their unit offsets when nbox > 1, unext: the queue head, zero): the cubes it
+// cannot take go to the boxes' group lists.
+void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, uint32_t *unext, uint32_t *stats,
+                   const LawTable &law, float rsphere, cudaStream_t st);
 WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &tb, float *ftree,
                  uint32_t *err);
 // One launch over the groups of every box (boxes: device array); the boxes

@@ -24,14 +24,13 @@
 #include <algorithm>
 
 #include "engine_internal.cuh"
+#include "short_range.cuh"
 
 namespace tpm {
 
 constexpr int kBuildThreads = 256;
 constexpr int kBuildGrid = 148 * 8;
 constexpr int kScanGrid = 148 * 2;
-
-TPM_D float wrapf(uint32_t a, uint32_t b, float cpu) { return (float)(int32_t)(a - b) * cpu; }
 
 // child boundary: first index in [lo, hi) whose digit at `shift` is >= d
 TPM_D uint32_t lower_digit(const uint64_t *key, uint32_t lo, uint32_t hi, int shift, uint32_t d) {
@@ -506,9 +505,20 @@ void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuff
   if (blocks > 148 * 16) blocks = 148 * 16;
   k_group_counts<<<blocks, 256, 0, st>>>(cube_start, ncubes, gcount, gmax);
   k_scan_block<<<(unsigned)nb, 1024, 0, st>>>(gcount, goff, ncubes, bsum);
-  k_scan_sums<<<1, 1024, 0, st>>>(bsum, nb, &tb.counters[0]);
+  k_scan_sums<<<1, 1024, 0, st>>>(bsum, nb, &tb.counters[kCntGroups]);
   k_write_groups<<<blocks, 256, 0, st>>>(cube_start, ncubes, goff, bsum, tb.groups, gmax);
   if (launches) *launches += 5;
+}
+
+void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
+                  cudaStream_t st, int64_t *launches) {
+  if (direct_applies(tp)) {
+    tree_units(tb, st, launches);
+  } else {
+    const int cbits = kAxisBits - tp.sub_bits;
+    tree_groups(tp, key, np, tb, cube_start, 1ll << (3 * (cbits - tp.group_level)), 3 * (tp.sub_bits + tp.group_level),
+                st, launches);
+  }
 }
 
 // ------------------------------------------------------------------ walk
@@ -519,7 +529,6 @@ constexpr int kStackSmem = 640;    // per-warp stack entries in shared memory
 constexpr int kStackCap = 8192;    // entries beyond kStackSmem live in global memory
 constexpr int kPcCap = 64;
 constexpr int kPpBatch = 128;       // particle sources evaluated per flush
-constexpr int kLogSmemF4 = (kLogEntries + 2) / 2;  // the log-spaced table, in float4s
 
 struct WarpLists {
   WalkBox box;                     // the box of the group this warp walks
@@ -540,70 +549,6 @@ struct WalkCtx {
   bool active;
   uint32_t rx, ry, rz;    // u_ref
 };
-
-// The law at s = r^2 + kLogR2Floor (cells^2) from the table indexed by the
-// float bits of s: the exponent and the top kLogMantissa mantissa bits pick
-// the bin, whose line in s gives the value, so neither a square root nor a
-// conversion is needed, and s >= 2^-20 needs no lower clamp. tlb is the
-// table's shared address with the base entry kLogBase folded in (s >= 2^-20
-// keeps the entry >= 0; the clamp keeps it in range).
-TPM_D float law_at(float s, uint32_t tlb) {
-  uint32_t kk = min(__float_as_uint(s) >> kLogShift, (uint32_t)(kLogBase + kLogEntries));
-  float2 c;
-  asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(c.x), "=f"(c.y) : "r"(tlb + (kk << 3)));
-  return fmaf(c.y, s, c.x);
-}
-
-// The law at s with every pair beyond the cut reading one shared entry: the
-// bin index is clamped at kcut (the first bin from which the Gaussian law's
-// table is zero; for the reference law the bin of rsphere^2, whose value the
-// per-pair test then discards), so the lanes with such pairs all load one
-// address, a broadcast, and the warp's gather spreads over the banks of the
-// pairs inside the cut only. Same value as law_at with the cut applied.
-TPM_D float law_clamped(float s, uint32_t tlb, uint32_t kcut) {
-  uint32_t kk = min(__float_as_uint(s) >> kLogShift, kcut);
-  float2 c;
-  asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(c.x), "=f"(c.y) : "r"(tlb + (kk << 3)));
-  return fmaf(c.y, s, c.x);
-}
-
-// One source against this lane's target: the reference's AddPar
-// (OST/ost.ver2.c:279-293) without the mass factor. The source comes negated
-// (nsx = -x), so dx = tx + nsx is the IEEE difference tx - x. The target
-// itself (r = 0) lands in bin 0 with a zero separation, adding nothing.
-// kHardCut: the per-pair cut of the reference law, tested as s <= rsphere^2
-// (a cut 2^-20 cells^2 inside r^2 <= rsphere^2); the Gaussian law's table is
-// zero from the cut on and needs no test.
-template <bool kHardCut>
-TPM_D void pp_one(float nsx, float nsy, float nsz, const WalkCtx &w, float rs2, uint32_t kcut, uint32_t tlb,
-                  float &ax, float &ay, float &az) {
-  float dx = w.tx + nsx, dy = w.ty + nsy, dz = w.tz + nsz;
-  float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, kLogR2Floor)));
-  float f = law_clamped(r2, tlb, kcut);
-  if (kHardCut) f = r2 <= rs2 ? f : 0.f;
-  ax = fmaf(dx, f, ax);
-  ay = fmaf(dy, f, ay);
-  az = fmaf(dz, f, az);
-}
-
-// Two sources against this lane's target, the separations, r^2 and the
-// accumulation as packed fp32x2 operations (sm_100 add/fma on register
-// pairs): each half is the IEEE fp32 operation pp_one does, in the same
-// order, so the sums are the same bits as two pp_one calls into the halves.
-template <bool kHardCut>
-TPM_D void pp_two(float2 nsx, float2 nsy, float2 nsz, float2 tx, float2 ty, float2 tz, float rs2, uint32_t kcut,
-                  uint32_t tlb, float2 &ax, float2 &ay, float2 &az) {
-  float2 dx = __fadd2_rn(tx, nsx), dy = __fadd2_rn(ty, nsy), dz = __fadd2_rn(tz, nsz);
-  float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(kLogR2Floor, kLogR2Floor))));
-  float2 f = make_float2(law_clamped(r2.x, tlb, kcut), law_clamped(r2.y, tlb, kcut));
-  if (kHardCut) {
-    f.x = r2.x <= rs2 ? f.x : 0.f;
-    f.y = r2.y <= rs2 ? f.y : 0.f;
-  }
-  ax = __ffma2_rn(dx, f, ax);
-  ay = __ffma2_rn(dy, f, ay);
-  az = __ffma2_rn(dz, f, az);
-}
 
 // The group's bounding box (cells, relative to u_ref) and the squared reach
 // beyond it: a source farther than that from the box is outside rsphere of
@@ -689,7 +634,7 @@ TPM_D void eval_pp(WarpLists &wl, int m, const uint32_t *__restrict__ spos, Walk
       z = zn;
     }
   }
-  for (; j < m; j++) pp_one<kHardCut>(nsx[j], nsy[j], nsz[j], w, rs2, kcut, tlb, a01x.x, a01y.x, a01z.x);
+  for (; j < m; j++) pp_one<kHardCut>(nsx[j], nsy[j], nsz[j], w.tx, w.ty, w.tz, rs2, kcut, tlb, a01x.x, a01y.x, a01z.x);
   if (w.active) {
     w.ax += (a01x.x + a01x.y) + (a23x.x + a23x.y);
     w.ay += (a01y.x + a01y.y) + (a23y.x + a23y.y);
@@ -773,38 +718,6 @@ TPM_D void eval_pc(WarpLists &wl, int m_all, const WalkBox &tb, WalkCtx &w, floa
   }
 }
 
-// The 4-cell cubes along one axis of an n-cell periodic box whose cells meet
-// [lo, hi] (cells, unwrapped): run[0..1] = first cube and count of the first
-// run, run[2..3] of the second (empty unless [lo, hi] wraps past n). Both
-// runs together list each cube once; an interval of n cells or more lists
-// every cube.
-TPM_D void axis_runs(float lo, float hi, int n, int run[4]) {
-  const int ncube = (n + 3) >> 2;
-  const float fn = (float)n;
-  run[0] = 0;
-  run[1] = ncube;
-  run[2] = 0;
-  run[3] = 0;
-  if (hi - lo >= fn) return;
-  float lw = lo - fn * floorf(lo / fn);
-  if (lw >= fn) lw = 0.f;
-  if (lw < 0.f) lw = 0.f;
-  float hw = lw + (hi - lo);
-  int a = min((int)(lw * 0.25f), ncube - 1);
-  if (hw < fn) {
-    int b = min((int)(hw * 0.25f), ncube - 1);
-    run[0] = a;
-    run[1] = b - a + 1;
-    return;
-  }
-  int b = min((int)((hw - fn) * 0.25f), ncube - 1);
-  if (b >= a) return;  // the runs meet: every cube
-  run[0] = a;
-  run[1] = ncube - a;
-  run[2] = 0;
-  run[3] = b + 1;
-}
-
 // The walk stack: the first kStackSmem entries in shared memory, the rest in
 // this warp's global region.
 struct WarpStack {
@@ -832,6 +745,8 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_tree_walk(
   float2 *tl = reinterpret_cast<float2 *>(smem4);
   float4 *tq = smem4 + kLogSmemF4;
   WarpLists *lists = reinterpret_cast<WarpLists *>(smem4 + kLogSmemF4 + kPcEntries + 1);
+  const uint32_t ngroups = nbox == 1 ? boxes[0].counters[kCntGroups] : gprefix[nbox];
+  if (ngroups == 0) return;  // the direct summation took every cube
   for (int i = threadIdx.x; i <= kLogEntries; i += kWalkThreads) tl[i] = glog[i];
   for (int i = threadIdx.x; i <= kPcEntries; i += kWalkThreads) tq[i] = gpc[i];
   __syncthreads();
@@ -839,7 +754,6 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_tree_walk(
   WarpLists &wl = lists[wib];
   int64_t gwarp = (int64_t)blockIdx.x * kWalkWarps + wib;
   WarpStack stack{wl.stack, stack_base + gwarp * (kStackCap - kStackSmem)};
-  const uint32_t ngroups = nbox == 1 ? *boxes[0].ngroups : gprefix[nbox];
   unsigned long long npp = 0, npc = 0, niter = 0, nvisit = 0;
   int max_top = 0;
   const uint32_t lanemask_lt = (1u << lane) - 1u;
@@ -1173,7 +1087,8 @@ WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &
   b.mom1 = tb.mom1;
   b.mom2 = tb.mom2;
   b.groups = tb.groups;
-  b.ngroups = tb.counters;  // counters[0] = the group count tree_groups wrote
+  b.units = tb.units;
+  b.counters = tb.counters;
   b.ftree = ftree;
   b.err = err;
   b.cube_node = tb.cube_node;
@@ -1182,7 +1097,7 @@ WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &
   b.mass = tp.mass;
   b.inv_ll = (float)(1.0 / ((double)tp.n * (double)tp.n));
   b.n_cells = (int)tp.n;
-  b.start_bits = kAxisBits - tp.sub_bits - 2;
+  b.group_max = std::max(1, std::min(32, tp.group_max));
   return b;
 }
 
@@ -1193,17 +1108,7 @@ static void launch_walk(const WalkBox *boxes, const uint32_t *gprefix, int nbox,
   int64_t max_grid = stack_words / ((int64_t)kWalkWarps * (kStackCap - kStackSmem));
   if (grid > max_grid) grid = (int)max_grid;
   const float rs2 = rsphere * rsphere;
-  // the bin every pair beyond the cut reads: for the reference law the bin
-  // of rsphere^2 (the per-pair test discards its value), for the Gaussian law
-  // the first bin of the table's zero tail
-  uint32_t kcut;
-  if (law.hard_cut) {
-    uint32_t b;
-    memcpy(&b, &rs2, 4);
-    kcut = b >> kLogShift;
-  } else {
-    kcut = law.cut_bits >> kLogShift;
-  }
+  const uint32_t kcut = law_cut_bin(law, rs2);
   if (law.hard_cut)
     k_tree_walk<true><<<grid, kWalkThreads, smem, st>>>(boxes, gprefix, nbox, gnext, stack, stats, law.tlog, law.tpc,
                                                         rs2, kcut);
@@ -1221,19 +1126,24 @@ void tree_walk(const TreeParams &tp, const uint32_t *spos, int64_t np, const Tre
   (void)np;
   // the box record goes to the device with the launch that precedes the walk
   k_set_walkbox<<<1, 32, 0, st>>>(tb.walkbox, walk_box(tp, spos, tb, ftree, err));
-  // tb.counters[1] is the next-group counter (zeroed before tree_groups)
-  launch_walk(tb.walkbox, nullptr, 1, &tb.counters[1], tb.stack, tb.stack_words, tb.counters, law, tp.rsphere, st);
+  // the next-item counters were zeroed before tree_groups / tree_units
+  if (direct_applies(tp)) {
+    launch_direct(tb.walkbox, nullptr, 1, &tb.counters[kCntNextUnit], tb.counters, law, tp.rsphere, st);
+    if (launches) *launches += 1;
+  }
+  launch_walk(tb.walkbox, nullptr, 1, &tb.counters[kCntNextGroup], tb.stack, tb.stack_words, tb.counters, law, tp.rsphere, st);
   if (launches) *launches += 2;
 }
 
-// Prefix of the boxes' group counts and the launch's next-group counter.
-__global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, uint32_t *__restrict__ gprefix,
+// Prefix of the boxes' group (or unit) counts, counters[word], and the
+// launch's next-item counter.
+__global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, int word, uint32_t *__restrict__ gprefix,
                                uint32_t *__restrict__ gnext) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     uint32_t run = 0;
     for (int b = 0; b < nbox; b++) {
       gprefix[b] = run;
-      run += *boxes[b].ngroups;
+      run += boxes[b].counters[word];
     }
     gprefix[nbox] = run;
     *gnext = 0;
@@ -1242,7 +1152,11 @@ __global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, uint
 
 void tree_walk_multi(const WalkBox *boxes, int nbox, uint32_t *gprefix, uint32_t *gnext, uint32_t *stack,
                      int64_t stack_words, uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st) {
-  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, gprefix, gnext);
+  // every box's direct summation first: it leaves the groups of the cubes it
+  // cannot take in the boxes' group lists
+  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntUnits, gprefix, gnext);
+  launch_direct(boxes, gprefix, nbox, gnext, stats, law, rsphere, st);
+  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntGroups, gprefix, gnext);
   launch_walk(boxes, gprefix, nbox, gnext, stack, stack_words, stats, law, rsphere, st);
 }
 

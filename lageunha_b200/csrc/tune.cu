@@ -60,16 +60,14 @@ TreeParams tree_params(const tpm_ctx *c) {
   tp.cell_per_unit = (float)((double)c->g.n / 4294967296.0);
   tp.mass = c->prm.particle_mass;
   tp.group_max = c->tune_group_max;
+  tp.group_level = c->tune_group_level;
   return tp;
 }
 
 void groups_and_walk(tpm_ctx *c) {
   TreeParams tp = tree_params(c);
-  const MeshGeom &g = c->g;
-  int glev = c->tune_group_level;
   cudaMemsetAsync(c->tb.counters, 0, sizeof(uint32_t) * 16, c->st);
-  tree_groups(tp, c->skey, c->np, c->tb, c->cube_start, 1ll << (3 * (g.cbits - glev)), 3 * (g.sub_bits + glev), c->st,
-              nullptr);
+  tree_targets(tp, c->skey, c->np, c->tb, c->cube_start, c->st, nullptr);
   tree_walk(tp, c->spos, c->np, c->tb, c->law, c->ftree, c->err, c->st, nullptr);
 }
 
