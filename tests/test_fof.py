@@ -53,3 +53,34 @@ def test_fof_singletons_and_no_groups():
         assert ng == 0 and np.all(lab == -1)
         with pytest.raises(E.EngineError):
             eng.fof(9.0, 2)                 # link of half the box
+
+
+def _set(kind, n):
+    """Positions for the cube search: clumps on the periodic corner and on
+    cube faces, dense enough for whole nodes to lie within the link, or a
+    sparse set with links across several cubes."""
+    rng = np.random.Generator(np.random.PCG64(77 + n))
+    if kind == "clumps":
+        c = np.array([[0, 0, 0], [4, 8, 4], [n - 1, 4, 0.02]], np.float64)
+        p = np.concatenate([c[i % 3] + 0.08 * rng.standard_normal((400, 3)) for i in range(3)] + [rng.random((300, 3)) * n])
+    else:
+        p = rng.random((500, 3)) * n
+    return ic.to_fixed_point(np.mod(p, n), n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,n,link,minm", [("clumps", 16, 0.2, 5), ("clumps", 45, 0.15, 2), ("clumps", 512, 0.25, 3),
+                                              ("sparse", 45, 3.0, 2), ("sparse", 16, 1.2, 1), ("sparse", 18, 5.0, 2)])
+def test_fof_cubes_and_cliques(kind, n, link, minm):
+    pu = _set(kind, n)
+    pos = ic.from_fixed_point(pu, n)
+    # no pair sits within the rounding of a 32-bit distance of the link
+    d = pos[:, None, :] - pos[None, :, :]
+    r = np.sqrt(((d - n * np.round(d / n)) ** 2).sum(-1))
+    assert np.min(np.abs(r - link)) > 2e-7 * link
+    want, ngw = O.fof_labels(n, pos, link, minm)
+    with E.Engine(n, epsilon=0.05) as eng:
+        eng.load_fixed(pu)
+        lab, ng = eng.fof(link, minm)
+    assert ng == ngw
+    assert np.array_equal(lab.astype(np.int64), want)
