@@ -577,25 +577,34 @@ __global__ void k_fft_cols(float2 *__restrict__ spec, float2 *__restrict__ spec2
                            const float2 *__restrict__ tw_n, int axis, float dir, int with_green, struct GreenArgs ga,
                            int TX, int nspec);
 
-cudaError_t fft_plan_init(FftPlan &p, int n, cudaStream_t st, DeviceArena *arena) {
+static int half_len(int n) { return n / 2 > 0 ? n / 2 : 1; }
+
+int64_t fft_twiddles(int n) { return (int64_t)n + half_len(n); }
+
+cudaError_t fft_plan_in(FftPlan &p, int n, float2 *tw, cudaStream_t st) {
   p.n = n;
-  p.arena = arena;
   const int max_smem = 160 * 1024;
   cudaFuncSetAttribute(k_fft_x_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   cudaFuncSetAttribute(k_fft_x_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   cudaFuncSetAttribute(k_fft_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-  int h = n / 2 > 0 ? n / 2 : 1;
-  cudaError_t e = dmalloc(arena, &p.tw, sizeof(float2) * n);
-  if (e == cudaSuccess) e = dmalloc(arena, &p.tw_half, sizeof(float2) * h);
-  if (e != cudaSuccess) return e;
+  int h = half_len(n);
+  p.tw = tw;
+  p.tw_half = tw + n;
   k_twiddles<<<(n + 255) / 256, 256, 0, st>>>(p.tw, n);
   k_twiddles<<<(h + 255) / 256, 256, 0, st>>>(p.tw_half, h);
   return cudaGetLastError();
 }
 
+cudaError_t fft_plan_init(FftPlan &p, int n, cudaStream_t st, DeviceArena *arena) {
+  p.arena = arena;
+  float2 *tw = nullptr;
+  cudaError_t e = dmalloc(arena, &tw, sizeof(float2) * fft_twiddles(n));
+  if (e != cudaSuccess) return e;
+  return fft_plan_in(p, n, tw, st);
+}
+
 void fft_plan_free(FftPlan &p) {
-  dfree(p.arena, p.tw);
-  dfree(p.arena, p.tw_half);
+  dfree(p.arena, p.tw);  // tw_half lies behind it
   p.tw = p.tw_half = nullptr;
 }
 
