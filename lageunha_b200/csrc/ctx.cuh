@@ -84,7 +84,6 @@ struct tpm_ctx {
   CUtensorMap tmap4b;
   float *gt = nullptr;       // tabulated influence function of the pair
   float gt_rs = -1.f;        // split scale gt was computed for
-  uint32_t *tile_start = nullptr;
   // tree
   tpm::TreeBuffers tb;
   uint32_t *cube_start = nullptr;

@@ -276,7 +276,6 @@ static void free_mesh(tpm_ctx *c) {
   dfree(c->arena, c->rho);
   dfree(c->arena, c->spec);
   dfree(c->arena, c->phi);
-  dfree(c->arena, c->tile_start);
   dfree(c->arena, c->cube_start);
   dfree(c->arena, c->tb.cube_node);
   dfree(c->arena, c->tb.start_cube);
@@ -286,7 +285,6 @@ static void free_mesh(tpm_ctx *c) {
   c->rho = nullptr;
   c->spec = nullptr;
   c->phi = nullptr;
-  c->tile_start = nullptr;
   c->cube_start = nullptr;
 }
 
@@ -301,8 +299,6 @@ static int alloc_mesh(tpm_ctx *c) {
   CK(dmalloc(c->arena, &c->spec, sizeof(float2) * g.spec_elems));
   CK(dmalloc(c->arena, &c->phi, sizeof(float) * (int64_t)g.px * g.py * g.pz));
   CK(cudaMemsetAsync(c->phi, 0, sizeof(float) * (int64_t)g.px * g.py * g.pz, c->st));
-  uint32_t ntiles = 1u << (3 * (g.cbits - 3));
-  CK(dmalloc(c->arena, &c->tile_start, sizeof(uint32_t) * (ntiles + 1)));
   c->ncubes = 1ll << (3 * (g.cbits - 2));
   CK(dmalloc(c->arena, &c->cube_start, sizeof(uint32_t) * (c->ncubes + 1)));
   c->tb.units = c->cube_start;
@@ -320,8 +316,7 @@ static int alloc_mesh(tpm_ctx *c) {
 
 static void free_particles(tpm_ctx *c) {
   void *ps[] = {c->pos, c->vel, c->key, c->key_alt, c->val, c->val_alt, c->spos, c->fpm, c->ftree, c->fout,
-                c->ss.hist, c->ss.dtotal, c->tb.start, c->tb.count, c->tb.child, c->tb.nchild, c->tb.level, c->tb.geo,
-                c->tb.mom0, c->tb.mom1, c->tb.mom2, c->tb.walkA, c->tb.walkB, c->tb.tile_sum, c->tb.groups};
+                c->ss.hist, c->ss.dtotal, c->tb.mom0, c->tb.mom1, c->tb.mom2, c->tb.walkA, c->tb.walkB, c->tb.tile_sum, c->tb.groups};
   quiesce(c);
   for (void *p : ps)
     dfree(c->arena, p);
@@ -333,9 +328,6 @@ static void free_particles(tpm_ctx *c) {
   c->fpm = c->ftree = c->fout = nullptr;
   c->ss.hist = nullptr;
   c->ss.dtotal = nullptr;
-  c->tb.start = c->tb.count = c->tb.child = c->tb.nchild = nullptr;
-  c->tb.level = nullptr;
-  c->tb.geo = nullptr;
   c->tb.mom0 = c->tb.mom1 = c->tb.mom2 = nullptr;
   c->tb.walkA = c->tb.walkB = nullptr;
   c->tb.tile_sum = nullptr;
@@ -368,20 +360,12 @@ static int ensure_particles(tpm_ctx *c, int64_t np) {
   int64_t cap_nodes = cap + cap / 4 + 64;
   TreeBuffers &tb = c->tb;
   tb.cap_nodes = cap_nodes;
-  CK(dmalloc(c->arena, &tb.start, sizeof(uint32_t) * cap_nodes));
-  CK(dmalloc(c->arena, &tb.count, sizeof(uint32_t) * cap_nodes));
-  CK(dmalloc(c->arena, &tb.child, sizeof(uint32_t) * cap_nodes));
-  CK(dmalloc(c->arena, &tb.nchild, sizeof(uint32_t) * cap_nodes));
-  CK(dmalloc(c->arena, &tb.level, sizeof(uint8_t) * cap_nodes));
-  CK(dmalloc(c->arena, &tb.geo, sizeof(uint4) * cap_nodes));
   CK(dmalloc(c->arena, &tb.mom0, sizeof(float4) * cap_nodes));
   CK(dmalloc(c->arena, &tb.mom1, sizeof(float4) * cap_nodes));
   CK(dmalloc(c->arena, &tb.mom2, sizeof(float4) * cap_nodes));
   CK(dmalloc(c->arena, &tb.walkA, sizeof(uint4) * 2 * cap_nodes));
   CK(dmalloc(c->arena, &tb.walkB, sizeof(uint4) * cap_nodes));
-  int64_t ts = (cap_nodes + 1023) / 1024 + 16;
-  int64_t need_groups = 2 * c->ncubes + (c->ncubes + 4095) / 4096 + 16;
-  if (ts < need_groups) ts = need_groups;
+  const int64_t ts = tree_scratch_words(cap, c->ncubes);
   tb.cap_tiles = ts;
   CK(dmalloc(c->arena, &tb.tile_sum, sizeof(uint32_t) * ts));
   tb.cap_groups = cap / 1 + c->ncubes + 16;
@@ -531,13 +515,12 @@ int64_t tpm::ctx_bytes(int n_mesh, int64_t np) {
   int64_t n3 = (int64_t)g.n * g.n * g.n;
   // both grids of the interlaced pair (the Gaussian law's second grid)
   int64_t mesh = 2 * (4 * n3 + 8 * g.spec_elems + 4 * (int64_t)g.px * g.py * g.pz) + 4 * g.spec_elems;
-  int64_t ntiles = 1ll << (3 * (g.cbits - 3)), ncubes = 1ll << (3 * (g.cbits - 2));
-  mesh += 4 * (ntiles + 1) + 3 * 4 * (ncubes + 1) + 8 * (int64_t)(n_mesh + n_mesh / 2 + 1);
+  int64_t ncubes = 1ll << (3 * (g.cbits - 2));
+  mesh += 3 * 4 * (ncubes + 1) + 8 * (int64_t)(n_mesh + n_mesh / 2 + 1);
   int64_t parts = np * (12 + 12 + 8 + 8 + 4 + 4 + 12 + 12 + 12 + 12) + 4 * 256 * (sort_tiles(np) + 1) + 1024;
   int64_t cap_nodes = np + np / 4 + 64;
-  int64_t tree = cap_nodes * (4 + 4 + 4 + 4 + 1 + 16 + 3 * 16 + 32 + 16);
-  int64_t ts = (cap_nodes + 1023) / 1024 + 16, need = 2 * ncubes + (ncubes + 4095) / 4096 + 16;
-  tree += 4 * (ts > need ? ts : need) + 8 * (np + ncubes + 16);
+  int64_t tree = cap_nodes * (3 * 16 + 32 + 16);
+  tree += 4 * tree_scratch_words(np, ncubes) + 8 * (np + ncubes + 16);
   int64_t fixed = 4 * walk_stack_words() + 8 * 4097 + 16 * 4096 + 4096;
   return mesh + parts + tree + fixed;
 }
@@ -778,7 +761,10 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
   c->skey = k;
   c->perm = v;
   launch_gather_pos(c->pos, c->perm, np, c->spos, st);
-  c->launches += 2;
+  // the particle ranges of the 4-cell cubes and, at every eighth entry, of the
+  // PM chain's 8-cell tiles
+  launch_range_table(c->skey, np, 3 * (g.sub_bits + 2), (uint32_t)c->tb.ncubes4, c->tb.start_cube, st);
+  c->launches += 3;
   CK(stage_check(st, "sort"));
   if (timing) CK(cudaEventRecord(c->ev[1], st));
   // ---- PM: with both parts, on st_pm beside the tree build
@@ -791,13 +777,11 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
     pst = c->st_pm;
   }
   if (parts & TPM_PART_PM) {
-    uint32_t ntiles = 1u << (3 * (g.cbits - 3));
-    launch_range_table(c->skey, np, 3 * (g.sub_bits + 3), ntiles, c->tile_start, pst);
     CK(cudaMemsetAsync(c->rho, 0, sizeof(float) * (int64_t)g.n * g.n * g.n, pst));
     const bool il = c->prm.law == TPM_LAW_GAUSSIAN;  // interlaced pair of grids
     if (il) CK(cudaMemsetAsync(c->rho2, 0, sizeof(float) * (int64_t)g.n * g.n * g.n, pst));
-    launch_tsc_deposit(g, c->spos, c->tile_start, c->prm.particle_mass, c->rho, pst, il ? c->rho2 : nullptr);
-    c->launches += 2;
+    launch_tsc_deposit(g, c->spos, c->tb.start_cube, c->prm.particle_mass, c->rho, pst, il ? c->rho2 : nullptr);
+    c->launches += il ? 2 : 1;
     CK(stage_check(pst, "deposit"));
     if (timing) CK(cudaEventRecord(c->ev[2], pst));
     double *pk = c->measure_pk ? c->pk_acc : nullptr;
@@ -813,10 +797,10 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
     // the reference law keeps the reference's 4-point gradient; the Gaussian
     // law uses the 8-point one on both interlaced grids and averages
     if (c->prm.law == TPM_LAW_REFERENCE) {
-      launch_fda4(g, &c->tmap2, 2, c->spos, c->tile_start, c->fpm, c->err, pst);
+      launch_fda4(g, &c->tmap2, 2, c->spos, c->tb.start_cube, c->fpm, c->err, pst);
       c->launches += 1;
     } else {
-      launch_fda4_pair(g, &c->tmap4, &c->tmap4b, c->spos, c->tile_start, c->fpm, c->err, pst);
+      launch_fda4_pair(g, &c->tmap4, &c->tmap4b, c->spos, c->tb.start_cube, c->fpm, c->err, pst);
       c->launches += 1;
     }
     CK(stage_check(pst, "fda4"));

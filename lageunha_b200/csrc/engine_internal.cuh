@@ -38,6 +38,8 @@ int64_t sort_tiles(int64_t np);
 void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, uint32_t *spos,
                        cudaStream_t st);
 // start[t] = first sorted index whose key >> shift >= t, t in [0, ntable].
+// (A Morton cube's eight sub-cubes are consecutive, so the table of the 4-cell
+// cubes at every eighth entry is that of the 8-cell tiles.)
 void launch_range_table(const uint64_t *key, int64_t np, int shift, uint32_t ntable, uint32_t *start,
                         cudaStream_t st);
 
@@ -58,7 +60,8 @@ MeshGeom make_geom(int n);
 
 // With rho2 the particles also go onto the second grid of the interlaced pair,
 // moved by half a cell along every axis (a second launch).
-void launch_tsc_deposit(const MeshGeom &g, const uint32_t *spos, const uint32_t *tile_start,
+// cube_start: the range table of the 4-cell cubes.
+void launch_tsc_deposit(const MeshGeom &g, const uint32_t *spos, const uint32_t *cube_start,
                         float mass, float *rho, cudaStream_t st, float *rho2 = nullptr);
 // Device memory arena (arena.cu): large blocks claimed from the driver once,
 // sub-ranges handed out best fit and merged back on release. Thread-safe.
@@ -117,12 +120,12 @@ void launch_green_opt(float *gt, int n, double rs, cudaStream_t st);
 // half: positions moved by half a cell (the shifted grid); average: write the
 // mean of the new force and the one already in fpm.
 void launch_fda4(const MeshGeom &g, const CUtensorMap *tmap, int radius, const uint32_t *spos,
-                 const uint32_t *tile_start, float *fpm, uint32_t *err, cudaStream_t st, int half = 0,
+                 const uint32_t *cube_start, float *fpm, uint32_t *err, cudaStream_t st, int half = 0,
                  int average = 0);
 // Both grids of the interlaced pair with the 8-point gradient in one pass:
 // fpm = the mean of the two grids' forces.
 void launch_fda4_pair(const MeshGeom &g, const CUtensorMap *tmap, const CUtensorMap *tmap2, const uint32_t *spos,
-                      const uint32_t *tile_start, float *fpm, uint32_t *err, cudaStream_t st);
+                      const uint32_t *cube_start, float *fpm, uint32_t *err, cudaStream_t st);
 // Tensor maps of the potential for the 4-point (radius 2) and the 8-point
 // (radius 4) gradient: their boxes differ.
 int make_phi_tensor_map(const MeshGeom &g, float *phi_pad, int radius, CUtensorMap *out);
@@ -162,19 +165,16 @@ enum TreeCounter : int {
 constexpr uint32_t kNoNode = 0xffffffffu;
 struct TreeBuffers {
   int64_t cap_nodes = 0;
-  uint32_t *start = nullptr, *count = nullptr, *child = nullptr, *nchild = nullptr;
-  uint8_t *level = nullptr;
-  uint4 *geo = nullptr;      // center u32 x3, half-size (float bits)
   float4 *mom0 = nullptr;    // com (u32 bits x3), mass
   float4 *mom1 = nullptr;    // Qxx Qyy Qzz Qxy
   float4 *mom2 = nullptr;    // Qxz Qyz trQ mass
-  // walk records, written with the moments: walkA[2n] = cube centre u32 x3 +
-  // half-size bits, walkA[2n+1] = com u32 x3 + size^2/theta^2 bits;
-  // walkB[n] = start, count, first child, nchild | level << 16
+  // walk records: walkA[2n] = cube centre u32 x3 + half-size bits, walkA[2n+1]
+  // = com u32 x3 + size^2/theta^2 bits; walkB[n] = start, count, first child,
+  // nchild | level << 16
   uint4 *walkA = nullptr;
   uint4 *walkB = nullptr;
   uint32_t *level_range = nullptr;  // [2*(kAxisBits+2)] begin/end per level
-  uint32_t *tile_sum = nullptr;     // scan scratch
+  uint32_t *tile_sum = nullptr;     // scan scratch (tree_scratch_words)
   int64_t cap_tiles = 0;
   uint32_t *groups = nullptr;       // walk groups: start | (count << 26) packed as 2 words
   int64_t cap_groups = 0;
@@ -213,6 +213,9 @@ void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuff
 inline bool direct_applies(const TreeParams &tp) {
   return tp.group_level == 2 && (float)tp.n >= 2.f * (4.f + tp.rsphere);
 }
+// Words of TreeBuffers::tile_sum: the build's counts per level and tile, or the
+// group counts and offsets of a mesh with ncubes 4-cell cubes.
+int64_t tree_scratch_words(int64_t np, int64_t ncubes);
 // What the short-range force iterates over: the units of the direct summation
 // where it applies, else every group of the tree walk.
 void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,

@@ -214,7 +214,7 @@ TPM_D void flush_tile(const uint32_t *acc, float inv_scale, float *__restrict__ 
 // a cell (the second grid of the interlaced pair). One grid per launch: a
 // kernel holding both grids' accumulators ran slower (fewer blocks per SM).
 __global__ void __launch_bounds__(kDepThreads) k_tsc_deposit(
-    const uint32_t *__restrict__ spos, const uint32_t *__restrict__ tile_start, int n, int cbits,
+    const uint32_t *__restrict__ spos, const uint32_t *__restrict__ cube_start, int n, int cbits,
     float mass, float *__restrict__ rho, uint32_t half, int vec4) {
   __shared__ __align__(16) uint32_t acc[kDepCells];
   int tid = threadIdx.x, lane = tid & 31;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kDepThreads) k_tsc_deposit(
     ty |= ((t >> (3 * b + 1)) & 1u) << b;
     tz |= ((t >> (3 * b + 2)) & 1u) << b;
   }
-  uint32_t p0 = tile_start[t], p1 = tile_start[t + 1];
+  uint32_t p0 = cube_start[8 * t], p1 = cube_start[8 * t + 8];
   if (p0 == p1) return;
   int ox = (int)tx * kTile - 1, oy = (int)ty * kTile - 1, oz = (int)tz * kTile - 1;
   for (int i = tid; i < kDepCells; i += kDepThreads) acc[i] = 0u;
@@ -272,12 +272,12 @@ __global__ void __launch_bounds__(kDepThreads) k_tsc_deposit(
   flush_tile(acc, inv_scale, rho, n, ox, oy, oz, vec4, tid);
 }
 
-void launch_tsc_deposit(const MeshGeom &g, const uint32_t *spos, const uint32_t *tile_start,
+void launch_tsc_deposit(const MeshGeom &g, const uint32_t *spos, const uint32_t *cube_start,
                         float mass, float *rho, cudaStream_t st, float *rho2) {
   uint32_t ntiles = 1u << (3 * (g.cbits - 3));
   int vec4 = (g.n % 4) == 0;
-  k_tsc_deposit<<<ntiles, kDepThreads, 0, st>>>(spos, tile_start, g.n, g.cbits, mass, rho, 0u, vec4);
-  if (rho2) k_tsc_deposit<<<ntiles, kDepThreads, 0, st>>>(spos, tile_start, g.n, g.cbits, mass, rho2, 1u, vec4);
+  k_tsc_deposit<<<ntiles, kDepThreads, 0, st>>>(spos, cube_start, g.n, g.cbits, mass, rho, 0u, vec4);
+  if (rho2) k_tsc_deposit<<<ntiles, kDepThreads, 0, st>>>(spos, cube_start, g.n, g.cbits, mass, rho2, 1u, vec4);
 }
 
 // ------------------------------------------------------------------ FFT
@@ -1279,7 +1279,7 @@ template <int R, bool kPair>
 __global__ void __launch_bounds__(kFdaThreads) k_fda4(const __grid_constant__ CUtensorMap tmap,
                                                       const __grid_constant__ CUtensorMap tmap2,
                                                       const uint32_t *__restrict__ spos,
-                                                      const uint32_t *__restrict__ tile_start, int n,
+                                                      const uint32_t *__restrict__ cube_start, int n,
                                                       int cbits, float *__restrict__ fpm,
                                                       uint32_t *__restrict__ err, uint32_t half, int average) {
   using B = FdaBox<R>;
@@ -1304,7 +1304,7 @@ __global__ void __launch_bounds__(kFdaThreads) k_fda4(const __grid_constant__ CU
     ty |= ((t >> (3 * b + 1)) & 1u) << b;
     tz |= ((t >> (3 * b + 2)) & 1u) << b;
   }
-  uint32_t p0 = tile_start[t], p1 = tile_start[t + 1];
+  uint32_t p0 = cube_start[8 * t], p1 = cube_start[8 * t + 8];
   if (p0 == p1) return;
   int x0 = (int)tx * kTile, y0 = (int)ty * kTile, z0 = (int)tz * kTile;
   if (tid == 0) {
@@ -1392,28 +1392,28 @@ int make_phi_tensor_map(const MeshGeom &g, float *phi_pad, int radius, CUtensorM
 }
 
 void launch_fda4(const MeshGeom &g, const CUtensorMap *tmap, int radius, const uint32_t *spos,
-                 const uint32_t *tile_start, float *fpm, uint32_t *err, cudaStream_t st, int half, int average) {
+                 const uint32_t *cube_start, float *fpm, uint32_t *err, cudaStream_t st, int half, int average) {
   uint32_t ntiles = 1u << (3 * (g.cbits - 3));
   const size_t nodes = sizeof(float) * 3 * kGradSize;
   if (radius == 2) {
     size_t smem = sizeof(float) * FdaBox<2>::BY * FdaBox<2>::BY * FdaBox<2>::BX + nodes;
     cudaFuncSetAttribute(k_fda4<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fda4<2, false><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap, spos, tile_start, g.n, g.cbits, fpm, err,
+    k_fda4<2, false><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap, spos, cube_start, g.n, g.cbits, fpm, err,
                                                         (uint32_t)half, average);
   } else {
     size_t smem = sizeof(float) * FdaBox<4>::BY * FdaBox<4>::BY * FdaBox<4>::BX + nodes;
     cudaFuncSetAttribute(k_fda4<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fda4<4, false><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap, spos, tile_start, g.n, g.cbits, fpm, err,
+    k_fda4<4, false><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap, spos, cube_start, g.n, g.cbits, fpm, err,
                                                         (uint32_t)half, average);
   }
 }
 
 void launch_fda4_pair(const MeshGeom &g, const CUtensorMap *tmap, const CUtensorMap *tmap2, const uint32_t *spos,
-                      const uint32_t *tile_start, float *fpm, uint32_t *err, cudaStream_t st) {
+                      const uint32_t *cube_start, float *fpm, uint32_t *err, cudaStream_t st) {
   uint32_t ntiles = 1u << (3 * (g.cbits - 3));
   size_t smem = sizeof(float) * FdaBox<4>::BY * FdaBox<4>::BY * FdaBox<4>::BX + 2 * sizeof(float) * 3 * kGradSize;
   cudaFuncSetAttribute(k_fda4<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_fda4<4, true><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap2, spos, tile_start, g.n, g.cbits, fpm, err, 0u, 0);
+  k_fda4<4, true><<<ntiles, kFdaThreads, smem, st>>>(*tmap, *tmap2, spos, cube_start, g.n, g.cbits, fpm, err, 0u, 0);
 }
 
 }  // namespace tpm

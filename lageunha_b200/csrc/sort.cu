@@ -266,14 +266,31 @@ void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, ui
   k_gather_pos<<<blocks, 256, 0, st>>>(pos, perm, np, spos);
 }
 
+// Thread i writes the entries (key[i - 1] >> shift, key[i] >> shift]. Where the
+// mesh is no power of two or particles are sparse, runs of empty entries are
+// long (thousands); those are written by the whole warp.
 __global__ void k_range_table(const uint64_t *__restrict__ key, int64_t np, int shift,
                               uint32_t ntable, uint32_t *__restrict__ start) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= np;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t t = i < np ? (int64_t)(key[i] >> shift) : (int64_t)ntable;
-    int64_t tp = i > 0 ? (int64_t)(key[i - 1] >> shift) : -1;
-    if (t > (int64_t)ntable) t = ntable;
-    for (int64_t q = tp + 1; q <= t; q++) start[q] = (uint32_t)i;
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); i0 <= np;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + lane;
+    int64_t t = -1, tp = -1;
+    if (i <= np) {
+      t = i < np ? (int64_t)(key[i] >> shift) : (int64_t)ntable;
+      tp = i > 0 ? (int64_t)(key[i - 1] >> shift) : -1;
+      if (t > (int64_t)ntable) t = ntable;
+    }
+    const bool longrun = t - tp > 8;
+    if (!longrun)
+      for (int64_t q = tp + 1; q <= t; q++) start[q] = (uint32_t)i;
+    unsigned m = __ballot_sync(0xffffffffu, longrun);
+    while (m) {
+      const int src = __ffs(m) - 1;
+      m &= m - 1;
+      const int64_t a = __shfl_sync(0xffffffffu, tp, src), b = __shfl_sync(0xffffffffu, t, src);
+      for (int64_t q = a + 1 + lane; q <= b; q += 32) start[q] = (uint32_t)(i0 + src);
+    }
   }
 }
 

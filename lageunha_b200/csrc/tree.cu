@@ -8,9 +8,9 @@
 // quadrupole node terms and particle terms from a tabulated law, both only
 // inside rsphere (ost.ver2.c:247-293; OST/Model4TreeForce.c:34-46).
 //
-// Here one octree covers the whole periodic box. It is built level by level
-// from the Morton-sorted keys (a node's children are the runs of its next
-// octal key digit), keeps the reference's leaf rule (children with fewer than
+// Here one octree covers the whole periodic box. It is built from the
+// Morton-sorted keys (a node's children are the runs of its next octal key
+// digit), keeps the reference's leaf rule (children with fewer than
 // 10 particles stay bare), and carries the same moments: mass, centre of
 // mass, second moments about it, trQ and size^2/theta^2. A warp walks the
 // tree for a group of up to 32 spatially adjacent targets, opening a node if
@@ -28,179 +28,163 @@
 
 namespace tpm {
 
-constexpr int kBuildThreads = 256;
 constexpr int kBuildGrid = 148 * 8;
-constexpr int kScanGrid = 148 * 2;
 
-// child boundary: first index in [lo, hi) whose digit at `shift` is >= d
-TPM_D uint32_t lower_digit(const uint64_t *key, uint32_t lo, uint32_t hi, int shift, uint32_t d) {
-  while (lo < hi) {
-    uint32_t mid = lo + ((hi - lo) >> 1);
-    uint32_t v = (uint32_t)(key[mid] >> shift) & 7u;
-    if (v < d)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
+// ------------------------------------------------------------------ nodes
+// A node is a cube that holds particles and whose parent holds at least
+// kLeafMin. In the sorted order it starts at the particle i whose key differs
+// from the one before it in a digit at or above the node's level, so every
+// particle's levels follow from the keys near it: with d the first level at
+// which key[i] differs from key[i - 1] and e(j) the last level at which key[j]
+// and key[j + kLeafMin - 1] agree,
+//   level d has a node at i if a run of kLeafMin particles around i shares the
+//   parent, max(e(j), i - kLeafMin < j <= i) >= d - 1, and
+//   each deeper level l has one if the level above, which also starts at i,
+//   holds kLeafMin, l <= e(i) + 1.
+// So all levels are found in two passes over the keys (count and write, with a
+// scan of the block counts per level between), where a level-by-level build
+// took four launches for each of the 13 levels: launch gaps at small particle
+// counts, and one binary search per child on every level. Nodes are ordered by
+// level, then by their first particle: the children of a node are contiguous.
+constexpr int kTbThreads = 256;
+constexpr int kTbWarps = kTbThreads / 32;
+constexpr int kTbBefore = kLeafMin;             // keys held before the tile
+constexpr int kTbLevels = kAxisBits + 2;        // levels 0..13 and one past
+// Particles per thread of a tile: a tile's chunks run one after another in
+// each warp, so small sets take short tiles for more warps in flight (32^3: 16
+// tiles of 8 per thread wrote the nodes in 38 us)
+constexpr int kTbItemsBig = 8, kTbItemsSmall = 1;
+inline int tb_items(int64_t np) { return np >= (1 << 20) ? kTbItemsBig : kTbItemsSmall; }
+
+int64_t tree_tiles(int64_t np) {
+  const int64_t tile = kTbThreads * tb_items(np);
+  return (np + tile - 1) / tile;
 }
 
-__global__ void k_tree_root(int64_t np, TreeBuffers tb, uint32_t n, int sub_bits) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    tb.start[0] = 0;
-    tb.count[0] = (uint32_t)np;
-    tb.child[0] = 0;
-    tb.nchild[0] = 0;
-    tb.level[0] = 0;
-    // root cube: [0, 2^(13-sub_bits)) cells, centre at half of that
-    double half = (double)(1u << (kAxisBits - 1)) / (double)(1u << sub_bits);
-    double cu = half / (double)n;
-    cu = cu - floor(cu);
-    uint32_t c = (uint32_t)(unsigned long long)llrint(cu * 4294967296.0);
-    tb.geo[0] = make_uint4(c, c, c, __float_as_uint((float)half));
-    for (int l = 0; l < 2 * (kAxisBits + 2); l++) tb.level_range[l] = 0;
-    tb.level_range[0] = 0;
-    tb.level_range[1] = 1;
-  }
+// The level at which two keys first differ (kAxisBits + 1 if they are equal).
+TPM_D int differ_level(uint64_t a, uint64_t b) {
+  uint64_t x = a ^ b;
+  if (!x) return kAxisBits + 1;
+  return kAxisBits - (63 - __clzll((long long)x)) / 3;
 }
 
-// The level kernels give each node a segment of 8 lanes, lane d owning the
-// node's d-th octant (its level-(l+1) digit): the eight child boundaries are
-// found by eight independent binary searches instead of one chain of seven,
-// and the children are written in parallel. Items are (node, digit) pairs;
-// the loops over them are warp-uniform, so the segment shuffles stay
-// converged.
-constexpr int kScanChunk = 4096;  // nodes per block of the per-level scan
-
-struct ChildRange {
-  uint32_t node;  // absolute index of the segment's node
-  bool valid;     // the node exists (item < 8 * nodes of the level)
-  uint32_t lo, hi;  // this lane's child [lo, hi), empty when the node does not split
+template <int kItems>
+struct TbShared {
+  static constexpr int kTile = kTbThreads * kItems;
+  static constexpr int kKeys = kTbBefore + kTile + kLeafMin;
+  uint64_t key[kKeys];           // keys [base - kTbBefore, base + tile + kLeafMin)
+  signed char e[kKeys];          // e(j) of the same slots, -1 where there is none
+  uint32_t wcnt[kTbWarps][kTbLevels + 1];
 };
 
-TPM_D ChildRange child_range(const uint64_t *__restrict__ key, const TreeBuffers &tb, uint32_t b,
-                             uint32_t nn, uint64_t item, int l, int shift) {
-  int d = threadIdx.x & 7;
-  ChildRange r;
-  r.valid = item < (uint64_t)nn * 8u;
-  r.node = b + (uint32_t)(item >> 3);
-  uint32_t s = 0, c = 0;
-  if (r.valid) {
-    s = tb.start[r.node];
-    c = tb.count[r.node];
+// The keys around the tile and their e(j), into shared memory.
+template <int kItems>
+TPM_D void tb_load(TbShared<kItems> &sm, const uint64_t *__restrict__ key, int64_t np, int64_t base) {
+  for (int t = threadIdx.x; t < sm.kKeys; t += kTbThreads) {
+    int64_t i = base - kTbBefore + t;
+    sm.key[t] = i >= 0 && i < np ? key[i] : 0ull;
   }
-  bool split = r.valid && c >= (uint32_t)kLeafMin && l < kAxisBits;
-  uint32_t bnd = s;
-  if (split && d > 0) bnd = lower_digit(key, s, s + c, shift, (uint32_t)d);
-  uint32_t nxt = __shfl_down_sync(0xffffffffu, bnd, 1, 8);
-  if (d == 7) nxt = s + c;
-  r.lo = bnd;
-  r.hi = split ? nxt : bnd;
-  return r;
+  __syncthreads();
+  for (int t = threadIdx.x; t < kTbBefore + sm.kTile; t += kTbThreads) {
+    int64_t i = base - kTbBefore + t;
+    sm.e[t] = (signed char)(i >= 0 && i + kLeafMin - 1 < np
+                                ? min(differ_level(sm.key[t], sm.key[t + kLeafMin - 1]) - 1, kAxisBits)
+                                : -1);
+  }
+  __syncthreads();
 }
 
-// Count the non-empty children of every level-l node that splits.
-__global__ void __launch_bounds__(kBuildThreads) k_tree_count(const uint64_t *__restrict__ key,
-                                                              TreeBuffers tb, int l) {
-  uint32_t b = tb.level_range[2 * l], e = tb.level_range[2 * l + 1];
-  uint32_t nn = e - b;
-  int lane = threadIdx.x & 31;
-  int shift = 3 * (kAxisBits - 1 - l);
-  const unsigned seg = 0xffu << (lane & ~7);
-  uint64_t total = (uint64_t)nn * 8u, stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-    ChildRange cr = child_range(key, tb, b, nn, base + lane, l, shift);
-    unsigned m = __ballot_sync(0xffffffffu, cr.hi > cr.lo) & seg;
-    if (cr.valid && (lane & 7) == 0) tb.nchild[cr.node] = (uint32_t)__popc(m);
+// The levels of the nodes that start at slot t (particle i), as a bit mask.
+template <int kItems>
+TPM_D uint32_t tb_levels(const TbShared<kItems> &sm, int t, int64_t i, int64_t np) {
+  if (i >= np) return 0u;
+  const int e = sm.e[t];
+  int first = 0;
+  if (i > 0) {
+    first = differ_level(sm.key[t], sm.key[t - 1]);
+    if (first > kAxisBits) return 0u;
+    int m = e;
+#pragma unroll
+    for (int q = 1; q < kLeafMin; q++) m = max(m, (int)sm.e[t - q]);
+    if (m < first - 1) return 0u;
+  }
+  const int last = max(first, min(kAxisBits, e + 1));
+  return (2u << last) - (1u << first);
+}
+
+// Nodes per level and tile: cnt[l * ntiles + tile].
+template <int kItems>
+__global__ void __launch_bounds__(kTbThreads) k_tree_count(const uint64_t *__restrict__ key, int64_t np,
+                                                           uint32_t *__restrict__ cnt, int64_t ntiles) {
+  __shared__ TbShared<kItems> sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t base = blockIdx.x * (int64_t)sm.kTile;
+  for (int q = lane; q < kTbLevels; q += 32) sm.wcnt[warp][q] = 0u;
+  tb_load(sm, key, np, base);
+#pragma unroll
+  for (int c = 0; c < kItems; c++) {
+    const int m = warp * (kItems * 32) + c * 32 + lane;
+    const uint32_t lv = tb_levels(sm, kTbBefore + m, base + m, np);
+    uint32_t any = __reduce_or_sync(0xffffffffu, lv);
+    while (any) {
+      const int l = __ffs(any) - 1;
+      any &= any - 1;
+      const unsigned b = __ballot_sync(0xffffffffu, (lv >> l) & 1u);
+      if (lane == 0) sm.wcnt[warp][l] += (uint32_t)__popc(b);
+    }
+  }
+  __syncthreads();
+  if (tid < kTbLevels) {
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < kTbWarps; w++) t += sm.wcnt[w][tid];
+    cnt[(int64_t)tid * ntiles + blockIdx.x] = t;
   }
 }
 
-// Per-level exclusive scan of nchild over chunks of kScanChunk nodes: the
-// prefix within the chunk goes to child[node] (the write pass adds the
-// chunk's offset and overwrites it), the chunk's total to tile_sum[chunk].
-__global__ void __launch_bounds__(1024) k_tree_scan_chunks(TreeBuffers tb, int l) {
+// One block per level: exclusive scan of the level's tile counts in place and
+// its total.
+__global__ void __launch_bounds__(1024) k_tree_scan(uint32_t *__restrict__ cnt, int64_t ntiles,
+                                                    uint32_t *__restrict__ total) {
   __shared__ uint32_t wsum[32];
-  uint32_t b = tb.level_range[2 * l], e = tb.level_range[2 * l + 1];
-  uint32_t nn = e - b;
-  uint32_t nchunks = (nn + kScanChunk - 1) / kScanChunk;
-  int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    uint32_t base = ch * kScanChunk;
+  uint32_t *h = cnt + (int64_t)blockIdx.x * ntiles;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t carry = 0;
+  for (int64_t base = 0; base < ntiles; base += 4096) {
     uint32_t v[4], s = 0;
+#pragma unroll
     for (int j = 0; j < 4; j++) {
-      uint32_t i = base + 4 * tid + j;
-      v[j] = i < nn ? tb.nchild[b + i] : 0u;
+      int64_t i = base + 4 * tid + j;
+      v[j] = i < ntiles ? h[i] : 0u;
       s += v[j];
     }
     uint32_t x = s;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) wsum[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      uint32_t t = wsum[lane];
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
-      }
-      wsum[lane] = t;
+    uint32_t w = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
     }
-    __syncthreads();
-    uint32_t run = (warp ? wsum[warp - 1] : 0u) + x - s;
+    const uint32_t all = __shfl_sync(0xffffffffu, w, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+    uint32_t run = carry + (warp ? before : 0u) + x - s;
+#pragma unroll
     for (int j = 0; j < 4; j++) {
-      uint32_t i = base + 4 * tid + j;
-      if (i < nn) tb.child[b + i] = run;
+      int64_t i = base + 4 * tid + j;
+      if (i < ntiles) h[i] = run;
       run += v[j];
     }
-    if (tid == 0) tb.tile_sum[ch] = wsum[31];
+    carry += all;
     __syncthreads();
   }
-}
-
-// Exclusive scan of the chunk sums of level l and the extent of level l+1.
-__global__ void __launch_bounds__(1024) k_tree_scan(TreeBuffers tb, int l, uint32_t *err) {
-  uint32_t b = tb.level_range[2 * l], e = tb.level_range[2 * l + 1];
-  uint32_t ntiles = (e - b + kScanChunk - 1) / kScanChunk;
-  __shared__ uint32_t wsum[32];
-  __shared__ uint32_t carry;
-  int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) carry = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < ntiles; base += 1024) {
-    uint32_t i = base + tid;
-    uint32_t v = i < ntiles ? tb.tile_sum[i] : 0u;
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t s = wsum[lane];
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += y;
-      }
-      wsum[lane] = s;
-    }
-    __syncthreads();
-    if (i < ntiles) tb.tile_sum[i] = carry + (warp ? wsum[warp - 1] : 0u) + x - v;
-    __syncthreads();
-    if (tid == 0) carry += wsum[31];
-    __syncthreads();
-  }
-  if (tid == 0) {
-    uint64_t end = (uint64_t)e + carry;
-    if (end > (uint64_t)tb.cap_nodes) {
-      atomicOr(err, (uint32_t)kErrNodeOverflow);
-      end = e;  // stop refining: the level's nodes stay leaves
-    }
-    tb.level_range[2 * (l + 1)] = e;
-    tb.level_range[2 * (l + 1) + 1] = (uint32_t)end;
-  }
+  if (tid == 0) total[blockIdx.x] = carry;
 }
 
 // The three axis coordinates interleaved in a Morton key (bit 3i + a of the
@@ -215,177 +199,349 @@ TPM_D uint32_t morton_compact(uint64_t x) {
   return (uint32_t)x;
 }
 
-// Write the children of level-l nodes: node records of level l+1 in the
-// order of their parents, siblings contiguous in octant order.
-// q_to_frac = 1 / (2^sub_bits n): axis units of the key to fractions of the
-// box, so a cube centre is one FP64 multiply (no divisions per node).
-__global__ void __launch_bounds__(kBuildThreads) k_tree_write(const uint64_t *__restrict__ key,
-                                                              TreeBuffers tb, int l, uint32_t n,
-                                                              int sub_bits, double q_to_frac) {
-  uint32_t b = tb.level_range[2 * l], e = tb.level_range[2 * l + 1];
-  uint32_t e1 = tb.level_range[2 * (l + 1) + 1];
-  bool overflow = (e1 == e);  // capacity hit: nothing written below this level
-  uint32_t nn = e - b;
-  int lane = threadIdx.x & 31;
-  int shift = 3 * (kAxisBits - 1 - l);
-  const unsigned seg = 0xffu << (lane & ~7);
-  int child_level = l + 1;
-  // child cube: side 2^(13-child_level) q units
-  uint32_t cside_q = 1u << (kAxisBits - child_level);
-  float half_cells = (float)((double)cside_q * 0.5 / (double)(1u << sub_bits));
-  uint64_t total = (uint64_t)nn * 8u, stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-    ChildRange cr = child_range(key, tb, b, nn, base + lane, l, shift);
-    bool ne = !overflow && cr.hi > cr.lo;
-    uint32_t first = 0;
-    if (cr.valid) first = e + tb.child[cr.node] + tb.tile_sum[(cr.node - b) / kScanChunk];
-    // every lane has read child[node] before the segment's lane 0 rewrites it
-    unsigned m = __ballot_sync(0xffffffffu, ne) & seg;
-    if (ne) {
-      uint32_t slot = first + (uint32_t)__popc(m & ((1u << lane) - 1u));
-      tb.start[slot] = cr.lo;
-      tb.count[slot] = cr.hi - cr.lo;
-      tb.child[slot] = 0;
-      tb.nchild[slot] = 0;
-      tb.level[slot] = (uint8_t)child_level;
-      // cube of the child from its first key
-      uint64_t k = key[cr.lo];
-      uint32_t q[3] = {morton_compact(k), morton_compact(k >> 1), morton_compact(k >> 2)};
+// The particles that share slot t's (particle i's) cube at level l, counted
+// from i: doubling steps and a binary search, in the tile's keys as far as
+// they reach.
+template <int kItems>
+TPM_D uint32_t tb_run(const TbShared<kItems> &sm, const uint64_t *__restrict__ key, int64_t np, int t, int64_t i, int l) {
+  const int shift = 3 * (kAxisBits - l);
+  const uint64_t mine = sm.key[t] >> shift;
+  auto same = [&](int64_t q) {
+    if (i + q >= np) return false;
+    return ((t + q < sm.kKeys ? sm.key[t + q] : key[i + q]) >> shift) == mine;
+  };
+  int64_t lo = 0, hi = 1;  // same(lo) holds
+  while (same(hi)) {
+    lo = hi;
+    hi *= 2;
+  }
+  while (hi - lo > 1) {
+    int64_t mid = (lo + hi) >> 1;
+    if (same(mid)) lo = mid;
+    else hi = mid;
+  }
+  return (uint32_t)hi;
+}
+
+// A node found by a warp, waiting to be written.
+struct TbNode {
+  uint32_t at;     // slot in the tile's keys << 8 | level
+  uint32_t node;   // its index
+  uint32_t below;  // the index its children start at
+};
+constexpr int kTbQueue = 64;
+
+// Writes every node's cube (walkA[2 node]), its first particle and count, the
+// index its children start at (for a node without children the index those of
+// the nodes after it start at) and its level (walkB[node]); the extents of the
+// levels; and the node of each 4-cell cube (cube_node, cleared to kNoNode
+// before). q_to_frac = 1 / (2^sub_bits n): axis units of the key to fractions
+// of the box. A quarter of the particles start a node, over several levels: a
+// warp queues the nodes it finds and writes them 32 at a time (written where
+// they were found, with a few lanes active, the pass took 648 us for 256^3
+// clustered particles).
+template <int kItems>
+__global__ void __launch_bounds__(kTbThreads) k_tree_write(const uint64_t *__restrict__ key, int64_t np, TreeBuffers tb,
+                                                           const uint32_t *__restrict__ cnt, int64_t ntiles,
+                                                           const uint32_t *__restrict__ total, int cube_level,
+                                                           int sub_bits, double q_to_frac, uint32_t *err) {
+  __shared__ TbShared<kItems> sm;
+  __shared__ TbNode queue[kTbWarps][kTbQueue];
+  __shared__ uint32_t lbase[kTbLevels + 1];  // first node of each level
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t base = blockIdx.x * (int64_t)sm.kTile;
+  for (int q = lane; q < kTbLevels + 1; q += 32) sm.wcnt[warp][q] = 0u;
+  if (tid == 0) {
+    uint32_t run = 0;
+    for (int l = 0; l <= kTbLevels; l++) {
+      lbase[l] = run;
+      if (l < kTbLevels) run += total[l];
+    }
+  }
+  tb_load(sm, key, np, base);
+  const bool fits = (int64_t)lbase[kTbLevels] <= tb.cap_nodes;
+  if (blockIdx.x == 0 && tid < kTbLevels) {
+    // past the capacity the tree keeps its root only
+    tb.level_range[2 * tid] = fits ? lbase[tid] : min(tid, 1);
+    tb.level_range[2 * tid + 1] = fits ? lbase[tid + 1] : 1u;
+    if (tid == 0 && !fits) atomicOr(err, (uint32_t)kErrNodeOverflow);
+  }
+  uint32_t lv[kItems];
+#pragma unroll
+  for (int c = 0; c < kItems; c++) {
+    const int m = warp * (kItems * 32) + c * 32 + lane;
+    lv[c] = tb_levels(sm, kTbBefore + m, base + m, np);
+    uint32_t any = __reduce_or_sync(0xffffffffu, lv[c]);
+    while (any) {
+      const int l = __ffs(any) - 1;
+      any &= any - 1;
+      const unsigned b = __ballot_sync(0xffffffffu, (lv[c] >> l) & 1u);
+      if (lane == 0) sm.wcnt[warp][l] += (uint32_t)__popc(b);
+    }
+  }
+  __syncthreads();
+  // each warp's first node of each level
+  if (tid < kTbLevels) {
+    uint32_t run = lbase[tid] + cnt[(int64_t)tid * ntiles + blockIdx.x];
+#pragma unroll
+    for (int w = 0; w < kTbWarps; w++) {
+      uint32_t t = sm.wcnt[w][tid];
+      sm.wcnt[w][tid] = run;
+      run += t;
+    }
+  }
+  __syncthreads();
+  const int cube_shift = 3 * (kAxisBits - cube_level);
+  // lane l keeps the index of the warp's next node of level l
+  uint32_t next = lane <= kTbLevels ? sm.wcnt[warp][lane] : 0u;
+  TbNode *wq = queue[warp];
+  int queued = 0;
+  auto write = [&](int count) {  // the first `count` nodes of the queue
+    if (lane < count) {
+      const TbNode e = wq[lane];
+      const int t = (int)(e.at >> 8), l = (int)(e.at & 0xffu);
+      const int64_t i = base + t - kTbBefore;
+      const uint64_t k = sm.key[t];
+      const uint32_t number = tb_run(sm, key, np, t, i, l);
+      const uint32_t side_q = 1u << (kAxisBits - l);
+      const uint32_t q[3] = {morton_compact(k), morton_compact(k >> 1), morton_compact(k >> 2)};
       uint32_t cu[3];
+#pragma unroll
       for (int a = 0; a < 3; a++) {
-        uint32_t qc = q[a] & ~(cside_q - 1u);
-        double fr = ((double)qc + 0.5 * (double)cside_q) * q_to_frac;
+        uint32_t qc = q[a] & ~(side_q - 1u);
+        double fr = ((double)qc + 0.5 * (double)side_q) * q_to_frac;
         fr -= floor(fr);
         cu[a] = (uint32_t)(unsigned long long)llrint(fr * 4294967296.0);
       }
-      tb.geo[slot] = make_uint4(cu[0], cu[1], cu[2], __float_as_uint(half_cells));
+      const float half_cells = (float)side_q * 0.5f / (float)(1u << sub_bits);
+      if ((int64_t)e.node < tb.cap_nodes) {
+        tb.walkA[2 * (int64_t)e.node] = make_uint4(cu[0], cu[1], cu[2], __float_as_uint(half_cells));
+        tb.walkB[e.node] = make_uint4((uint32_t)i, number, e.below, (uint32_t)l << 16);
+        if (l == cube_level) tb.cube_node[k >> cube_shift] = e.node;
+      }
     }
-    if (cr.valid && (lane & 7) == 0) {
-      tb.child[cr.node] = m ? first : 0u;
-      if (overflow) tb.nchild[cr.node] = 0;
+  };
+#pragma unroll
+  for (int c = 0; c < kItems; c++) {
+    const int m = warp * (kItems * 32) + c * 32 + lane;
+    const uint32_t any = __reduce_or_sync(0xffffffffu, lv[c]);
+    if (any) {
+      // from the deepest level of the chunk up: `below` is the index of the
+      // first node of the level below that starts at this particle or after it
+      const int top = 31 - __clz(any), low = __ffs(any) - 1;
+      uint32_t below = __shfl_sync(0xffffffffu, next, top + 1);
+      for (int l = top; l >= low; l--) {
+        const bool mine = (lv[c] >> l) & 1u;
+        const unsigned b = __ballot_sync(0xffffffffu, mine);
+        const uint32_t run = __shfl_sync(0xffffffffu, next, l);
+        const uint32_t before = (uint32_t)__popc(b & ((1u << lane) - 1u)), node = run + before;
+        if (lane == l) next += (uint32_t)__popc(b);
+        if (mine) wq[queued + before] = TbNode{(uint32_t)(kTbBefore + m) << 8 | (uint32_t)l, node, below};
+        queued += __popc(b);
+        below = node;
+        __syncwarp();
+        if (queued >= 32) {
+          write(32);
+          __syncwarp();
+          TbNode rest;
+          if (lane + 32 < queued) rest = wq[lane + 32];
+          __syncwarp();
+          if (lane + 32 < queued) wq[lane] = rest;
+          queued -= 32;
+          __syncwarp();
+        }
+      }
     }
+  }
+  write(queued);
+}
+
+int64_t tree_scratch_words(int64_t np, int64_t ncubes) {
+  // tree_tiles of the capacity's and of every smaller particle count
+  const int64_t tiles = std::max(tree_tiles(np), tree_tiles(std::min<int64_t>(np, (1 << 20) - 1)));
+  return std::max<int64_t>(kTbLevels * (tiles + 1), 2 * ncubes + (ncubes + 4095) / 4096) + 16;
+}
+
+// Moments of a node: mass, centre of mass (cells, relative to the cube's
+// centre), second moments about it and the squared size, which is max |x -
+// com| for leaves and the bound max_c(|com_c - com| + size_c) for inner nodes.
+struct NodeMoments {
+  float M, cx, cy, cz, qxx, qyy, qzz, qxy, qxz, qyz, size2;
+};
+
+TPM_D void put_moments(const TreeBuffers &tb, uint32_t node, uint4 geo, const NodeMoments &m, float cpu, float inv_theta2) {
+  uint32_t comx = geo.x + (uint32_t)(int32_t)__float2int_rn(m.cx / cpu);
+  uint32_t comy = geo.y + (uint32_t)(int32_t)__float2int_rn(m.cy / cpu);
+  uint32_t comz = geo.z + (uint32_t)(int32_t)__float2int_rn(m.cz / cpu);
+  tb.mom0[node] = make_float4(__uint_as_float(comx), __uint_as_float(comy), __uint_as_float(comz), m.M);
+  tb.mom1[node] = make_float4(m.qxx, m.qyy, m.qzz, m.qxy);
+  tb.mom2[node] = make_float4(m.qxz, m.qyz, m.qxx + m.qyy + m.qzz, m.M);
+  tb.walkA[2 * (int64_t)node + 1] = make_uint4(comx, comy, comz, __float_as_uint(m.size2 * inv_theta2));
+}
+
+// Every node's number of children (the difference of the next node's first
+// child index and its own; 0 for a node that does not split), and the moments
+// of those without, from their particles.
+__global__ void __launch_bounds__(256) k_tree_leaves(const uint32_t *__restrict__ spos, TreeBuffers tb, float cpu,
+                                                     float mass, float inv_theta2) {
+  __shared__ uint32_t lr[2 * kTbLevels];
+  if (threadIdx.x < 2 * kTbLevels) lr[threadIdx.x] = tb.level_range[threadIdx.x];
+  __syncthreads();
+  uint32_t nodes = 0;
+  for (int l = 0; l < kTbLevels; l++) nodes = max(nodes, lr[2 * l + 1]);
+  for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < nodes; node += gridDim.x * blockDim.x) {
+    const uint4 rec = tb.walkB[node];
+    const int l = (int)(rec.w >> 16);
+    const uint32_t s = rec.x, c = rec.y;
+    if (c >= (uint32_t)kLeafMin && l < kAxisBits) {
+      const uint32_t next = node + 1 < lr[2 * l + 1] ? tb.walkB[node + 1].z : lr[2 * (l + 1) + 1];
+      reinterpret_cast<uint32_t *>(&tb.walkB[node])[3] = (next - rec.z) | ((uint32_t)l << 16);
+      continue;
+    }
+    const uint4 geo = tb.walkA[2 * (int64_t)node];
+    NodeMoments m;
+    float sx = 0, sy = 0, sz = 0;
+    for (uint32_t i = s; i < s + c; i++) {
+      sx += wrapf(spos[3 * (int64_t)i + 0], geo.x, cpu);
+      sy += wrapf(spos[3 * (int64_t)i + 1], geo.y, cpu);
+      sz += wrapf(spos[3 * (int64_t)i + 2], geo.z, cpu);
+    }
+    float inv = 1.f / (float)c;
+    m.cx = sx * inv;
+    m.cy = sy * inv;
+    m.cz = sz * inv;
+    m.M = mass * (float)c;
+    m.qxx = m.qyy = m.qzz = m.qxy = m.qxz = m.qyz = m.size2 = 0.f;
+    for (uint32_t i = s; i < s + c; i++) {
+      float dx = wrapf(spos[3 * (int64_t)i + 0], geo.x, cpu) - m.cx;
+      float dy = wrapf(spos[3 * (int64_t)i + 1], geo.y, cpu) - m.cy;
+      float dz = wrapf(spos[3 * (int64_t)i + 2], geo.z, cpu) - m.cz;
+      m.qxx += mass * dx * dx;
+      m.qyy += mass * dy * dy;
+      m.qzz += mass * dz * dz;
+      m.qxy += mass * dx * dy;
+      m.qxz += mass * dx * dz;
+      m.qyz += mass * dy * dz;
+      m.size2 = fmaxf(m.size2, dx * dx + dy * dy + dz * dz);
+    }
+    put_moments(tb, node, geo, m, cpu, inv_theta2);
   }
 }
 
-// Moments of level-l nodes: leaves from their particles, inner nodes from
-// their children (parallel-axis theorem). size is max |x - com| for leaves
-// and the bound max_c(|com_c - com| + size_c) for inner nodes.
-__global__ void __launch_bounds__(256) k_tree_moments(const uint32_t *__restrict__ spos, TreeBuffers tb,
-                                                      int l, float cpu, float mass, float inv_theta2) {
-  uint32_t b = tb.level_range[2 * l], e = tb.level_range[2 * l + 1];
-  for (uint32_t node = b + blockIdx.x * blockDim.x + threadIdx.x; node < e;
-       node += gridDim.x * blockDim.x) {
-    uint4 geo = tb.geo[node];
-    uint32_t nch = tb.nchild[node];
-    float M = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-    float qxx = 0, qyy = 0, qzz = 0, qxy = 0, qxz = 0, qyz = 0, size2 = 0.f;
-    if (nch == 0) {
-      uint32_t s = tb.start[node], c = tb.count[node];
-      float sx = 0, sy = 0, sz = 0;
-      for (uint32_t i = s; i < s + c; i++) {
-        sx += wrapf(spos[3 * (int64_t)i + 0], geo.x, cpu);
-        sy += wrapf(spos[3 * (int64_t)i + 1], geo.y, cpu);
-        sz += wrapf(spos[3 * (int64_t)i + 2], geo.z, cpu);
-      }
-      float inv = 1.f / (float)c;
-      cx = sx * inv;
-      cy = sy * inv;
-      cz = sz * inv;
-      M = mass * (float)c;
-      for (uint32_t i = s; i < s + c; i++) {
-        float dx = wrapf(spos[3 * (int64_t)i + 0], geo.x, cpu) - cx;
-        float dy = wrapf(spos[3 * (int64_t)i + 1], geo.y, cpu) - cy;
-        float dz = wrapf(spos[3 * (int64_t)i + 2], geo.z, cpu) - cz;
-        qxx += mass * dx * dx;
-        qyy += mass * dy * dy;
-        qzz += mass * dz * dz;
-        qxy += mass * dx * dy;
-        qxz += mass * dx * dz;
-        qyz += mass * dy * dz;
-        size2 = fmaxf(size2, dx * dx + dy * dy + dz * dz);
-      }
-    } else {
-      uint32_t c0 = tb.child[node];
-      for (uint32_t j = c0; j < c0 + nch; j++) {
-        float4 m0 = tb.mom0[j];
-        float m = m0.w;
-        float dx = wrapf(__float_as_uint(m0.x), geo.x, cpu);
-        float dy = wrapf(__float_as_uint(m0.y), geo.y, cpu);
-        float dz = wrapf(__float_as_uint(m0.z), geo.z, cpu);
-        M += m;
-        cx += m * dx;
-        cy += m * dy;
-        cz += m * dz;
-      }
-      float inv = 1.f / M;
-      cx *= inv;
-      cy *= inv;
-      cz *= inv;
-      float size = 0.f;
-      for (uint32_t j = c0; j < c0 + nch; j++) {
-        float4 m0 = tb.mom0[j], m1 = tb.mom1[j], m2 = tb.mom2[j];
-        float child_open2 = __uint_as_float(tb.walkA[2 * (int64_t)j + 1].w);
-        float m = m0.w;
-        float dx = wrapf(__float_as_uint(m0.x), geo.x, cpu) - cx;
-        float dy = wrapf(__float_as_uint(m0.y), geo.y, cpu) - cy;
-        float dz = wrapf(__float_as_uint(m0.z), geo.z, cpu) - cz;
-        qxx += m1.x + m * dx * dx;
-        qyy += m1.y + m * dy * dy;
-        qzz += m1.z + m * dz * dz;
-        qxy += m1.w + m * dx * dy;
-        qxz += m2.x + m * dx * dz;
-        qyz += m2.y + m * dy * dz;
-        // child size from its open2 = size^2/theta^2
-        float cs = sqrtf(child_open2 / inv_theta2);
-        size = fmaxf(size, sqrtf(dx * dx + dy * dy + dz * dz) + cs);
-      }
-      size2 = size * size;
+// The moments of the level's nodes [b, e) that have children, from those
+// (parallel-axis theorem): eight lanes per node, one child each, so a node
+// takes one round of loads; `at` of `step` segments of eight lanes. Called by
+// whole warps.
+TPM_D void inner_moments(const TreeBuffers &tb, uint32_t b, uint32_t e, uint32_t at, uint32_t step, float cpu,
+                         float inv_theta2) {
+  const int d = threadIdx.x & 7;
+  auto sum8 = [](float v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  const uint32_t warp_at = at - ((threadIdx.x & 31) >> 3);  // the first segment of this warp
+  for (uint32_t n0 = b + warp_at; n0 < e; n0 += step) {
+    const uint32_t node = n0 + ((threadIdx.x & 31) >> 3);
+    uint4 rec = make_uint4(0, 0, 0, 0);
+    if (node < e) rec = tb.walkB[node];
+    const uint32_t nch = rec.w & 0xffffu;
+    if (__all_sync(0xffffffffu, nch == 0)) continue;
+    uint4 geo = make_uint4(0, 0, 0, 0);
+    float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0;
+    float open2 = 0.f;
+    if (nch) geo = tb.walkA[2 * (int64_t)node];
+    const bool on = (uint32_t)d < nch;
+    if (on) {
+      const int64_t j = (int64_t)rec.z + d;
+      m0 = tb.mom0[j];
+      m1 = tb.mom1[j];
+      m2 = tb.mom2[j];
+      open2 = __uint_as_float(tb.walkA[2 * j + 1].w);
     }
-    uint32_t comx = geo.x + (uint32_t)(int32_t)__float2int_rn(cx / cpu);
-    uint32_t comy = geo.y + (uint32_t)(int32_t)__float2int_rn(cy / cpu);
-    uint32_t comz = geo.z + (uint32_t)(int32_t)__float2int_rn(cz / cpu);
-    tb.mom0[node] = make_float4(__uint_as_float(comx), __uint_as_float(comy), __uint_as_float(comz), M);
-    tb.mom1[node] = make_float4(qxx, qyy, qzz, qxy);
-    tb.mom2[node] = make_float4(qxz, qyz, qxx + qyy + qzz, M);
-    tb.walkA[2 * (int64_t)node] = geo;
-    tb.walkA[2 * (int64_t)node + 1] = make_uint4(comx, comy, comz, __float_as_uint(size2 * inv_theta2));
-    tb.walkB[node] = make_uint4(tb.start[node], tb.count[node], tb.child[node],
-                                nch | ((uint32_t)tb.level[node] << 16));
+    float dx = 0.f, dy = 0.f, dz = 0.f;
+    if (on) {
+      dx = wrapf(__float_as_uint(m0.x), geo.x, cpu);
+      dy = wrapf(__float_as_uint(m0.y), geo.y, cpu);
+      dz = wrapf(__float_as_uint(m0.z), geo.z, cpu);
+    }
+    const float w = m0.w;
+    NodeMoments m;
+    m.M = sum8(w);
+    const float inv = nch ? 1.f / m.M : 0.f;
+    m.cx = sum8(w * dx) * inv;
+    m.cy = sum8(w * dy) * inv;
+    m.cz = sum8(w * dz) * inv;
+    dx -= m.cx;
+    dy -= m.cy;
+    dz -= m.cz;
+    m.qxx = sum8(on ? m1.x + w * dx * dx : 0.f);
+    m.qyy = sum8(on ? m1.y + w * dy * dy : 0.f);
+    m.qzz = sum8(on ? m1.z + w * dz * dz : 0.f);
+    m.qxy = sum8(on ? m1.w + w * dx * dy : 0.f);
+    m.qxz = sum8(on ? m2.x + w * dx * dz : 0.f);
+    m.qyz = sum8(on ? m2.y + w * dy * dz : 0.f);
+    // child size from its open2 = size^2/theta^2
+    float size = on ? sqrtf(dx * dx + dy * dy + dz * dz) + sqrtf(open2 / inv_theta2) : 0.f;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) size = fmaxf(size, __shfl_xor_sync(0xffffffffu, size, o));
+    m.size2 = size * size;
+    if (nch && d == 0) put_moments(tb, node, geo, m, cpu, inv_theta2);
   }
 }
 
-// The walk's start table: the node of every 4-cell cube at tree level
-// cbits - 2 (the table was cleared to kNoNode before).
-__global__ void k_cube_nodes(const uint64_t *__restrict__ key, TreeBuffers tb, int lev, int shift) {
-  uint32_t b = tb.level_range[2 * lev], e = tb.level_range[2 * lev + 1];
-  for (uint32_t node = b + blockIdx.x * blockDim.x + threadIdx.x; node < e; node += gridDim.x * blockDim.x)
-    tb.cube_node[key[tb.start[node]] >> shift] = node;
+__global__ void __launch_bounds__(256) k_tree_inner(TreeBuffers tb, int l, float cpu, float inv_theta2) {
+  inner_moments(tb, tb.level_range[2 * l], tb.level_range[2 * l + 1], (blockIdx.x * blockDim.x + threadIdx.x) >> 3,
+                (gridDim.x * blockDim.x) >> 3, cpu, inv_theta2);
+}
+
+// Levels lmax to 0 in one launch, one cluster of kTopBlocks blocks with its
+// hardware barrier between the levels.
+constexpr int kTopBlocks = 8;
+constexpr int kTopThreads = 512;
+__global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads)
+    k_tree_top(TreeBuffers tb, int lmax, float cpu, float inv_theta2) {
+  for (int l = lmax; l >= 0; l--) {
+    inner_moments(tb, tb.level_range[2 * l], tb.level_range[2 * l + 1], (blockIdx.x * kTopThreads + threadIdx.x) >> 3,
+                  (kTopBlocks * kTopThreads) >> 3, cpu, inv_theta2);
+    __threadfence();
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
 }
 
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
                 TreeBuffers &tb, uint32_t *err, cudaStream_t st, int64_t *launches) {
-  k_tree_root<<<1, 32, 0, st>>>(np, tb, tp.n, tp.sub_bits);
-  int64_t nl = 1;
-  for (int l = 0; l < kAxisBits; l++) {
-    k_tree_count<<<kBuildGrid, kBuildThreads, 0, st>>>(key, tb, l);
-    k_tree_scan_chunks<<<kScanGrid, 1024, 0, st>>>(tb, l);
-    k_tree_scan<<<1, 1024, 0, st>>>(tb, l, err);
-    k_tree_write<<<kBuildGrid, kBuildThreads, 0, st>>>(key, tb, l, tp.n, tp.sub_bits,
-                                                       1.0 / ((double)(1u << tp.sub_bits) * (double)tp.n));
-    nl += 4;
-  }
+  const int cbits = kAxisBits - tp.sub_bits;
+  const int64_t ntiles = tree_tiles(np);
+  uint32_t *cnt = tb.tile_sum, *total = cnt + kTbLevels * ntiles;
+  cudaMemsetAsync(tb.cube_node, 0xff, sizeof(uint32_t) * tb.ncubes4, st);
+  const double q_to_frac = 1.0 / ((double)(1u << tp.sub_bits) * (double)tp.n);
+  const bool big = tb_items(np) == kTbItemsBig;
+  if (big)
+    k_tree_count<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
+  else
+    k_tree_count<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
+  k_tree_scan<<<kTbLevels, 1024, 0, st>>>(cnt, ntiles, total);
+  if (big)
+    k_tree_write<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
+                                                                       tp.sub_bits, q_to_frac, err);
+  else
+    k_tree_write<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
+                                                                         tp.sub_bits, q_to_frac, err);
   float inv_theta2 = 1.f / tp.theta2;
-  for (int l = kAxisBits; l >= 0; l--) {
-    k_tree_moments<<<kBuildGrid, 256, 0, st>>>(spos, tb, l, tp.cell_per_unit, tp.mass, inv_theta2);
+  const int leaf_grid = (int)std::min<int64_t>((np + 255) / 256, kBuildGrid);
+  k_tree_leaves<<<leaf_grid, 256, 0, st>>>(spos, tb, tp.cell_per_unit, tp.mass, inv_theta2);
+  int64_t nl = 4;
+  // the levels of at most 8 nodes per segment of the cluster in one launch,
+  // each deeper one in its own
+  int l = kAxisBits - 1;
+  for (; l > 4; l--) {
+    k_tree_inner<<<(int)std::min<int64_t>((np + 31) / 32, kBuildGrid), 256, 0, st>>>(tb, l, tp.cell_per_unit, inv_theta2);
     nl++;
   }
-  // the walk's start tables over the 4-cell cubes
-  const int cbits = kAxisBits - tp.sub_bits;
-  const int shift = 3 * (tp.sub_bits + 2);
-  launch_range_table(key, np, shift, (uint32_t)tb.ncubes4, tb.start_cube, st);
-  cudaMemsetAsync(tb.cube_node, 0xff, sizeof(uint32_t) * tb.ncubes4, st);
-  k_cube_nodes<<<kBuildGrid, 256, 0, st>>>(key, tb, cbits - 2, shift);
-  nl += 3;
+  k_tree_top<<<kTopBlocks, kTopThreads, 0, st>>>(tb, l, tp.cell_per_unit, inv_theta2);
+  nl++;
   if (launches) *launches += nl;
 }
 
