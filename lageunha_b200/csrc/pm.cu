@@ -296,28 +296,21 @@ struct Factors {
 // (enough bytes in flight per SM for the transposing passes to stream)
 constexpr int kLoadBatch = 8;
 
-// radices of the x passes (packed rows) and of the column passes
-constexpr int kXRadixMax = 16;
-constexpr int kColRadixMax = 16;
-
-static Factors factorize(int L, int rmax) {
+// Radices of a length-L transform, the power of two first, cut into as few and
+// as even radices up to 16 as it takes: 512 = 8 x 8 x 8, where 16 x 16 x 2 spends
+// a whole pass through shared memory on butterflies of two.
+static Factors factorize(int L) {
   Factors f;
   f.nf = 0;
-  while (rmax >= 16 && L % 16 == 0) {
-    f.r[f.nf++] = 16;
-    L /= 16;
-  }
-  if (rmax >= 8 && L % 8 == 0) {
-    f.r[f.nf++] = 8;
-    L /= 8;
-  }
-  while (L % 4 == 0) {
-    f.r[f.nf++] = 4;
-    L /= 4;
-  }
+  int k = 0;
   while (L % 2 == 0) {
-    f.r[f.nf++] = 2;
+    k++;
     L /= 2;
+  }
+  for (int stages = (k + 3) / 4; stages > 0; stages--) {
+    int e = (k + stages - 1) / stages;
+    f.r[f.nf++] = 1 << e;
+    k -= e;
   }
   while (L % 3 == 0) {
     f.r[f.nf++] = 3;
@@ -337,17 +330,20 @@ static Factors factorize(int L, int rmax) {
 struct Div {
   int d, s;     // s >= 0: d == 1 << s
   float inv;
-  TPM_D int q(int e) const {
+  TPM_HD int q(int e) const {
     if (s >= 0) return e >> s;
     int p = (int)((float)e * inv);
     int r = e - p * d;
     return r < 0 ? p - 1 : (r >= d ? p + 1 : p);
   }
 };
-TPM_D Div make_div(int d) {
+static Div make_div(int d) {
   Div r;
   r.d = d;
-  r.s = (d & (d - 1)) == 0 ? __ffs(d) - 1 : -1;
+  r.s = -1;
+  if ((d & (d - 1)) == 0)
+    for (r.s = 0; (1 << r.s) < d; r.s++) {
+    }
   r.inv = r.s >= 0 ? 0.f : 1.f / (float)d;
   return r;
 }
@@ -478,27 +474,29 @@ TPM_D void dft_small<16>(float2 *v, float dir) {
   }
 }
 
+// dj, dn: the quotients by L / R and Ns. In the first stage (Ns = 1) every
+// twiddle is one.
 template <int R>
-TPM_D void stockham_stage(const float2 *in, float2 *out, const float2 *tw, int L, int ld, int Ns, int P,
-                          float dir, int tid, int nth) {
-  int jobs_per = L / R;
-  int step = L / (Ns * R);
+TPM_D void stockham_stage(const float2 *in, float2 *out, const float2 *tw, int L, int ld, int Ns, int P, float dir,
+                          const Div &dj, const Div &dn, int tid, int nth) {
+  const int jobs_per = dj.d;
+  const int step = dn.q(jobs_per);
   for (int job = tid; job < P * jobs_per; job += nth) {
-    int p = job / jobs_per, j = job - p * jobs_per;
+    int p = dj.q(job), j = job - p * jobs_per;
     const float2 *src = in + p * ld;
     float2 *dst = out + p * ld;
-    int jn = j / Ns;
+    int jn = dn.q(j);
     int k = j - jn * Ns;
     float2 v[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      float2 x = src[fslot(j + r * jobs_per)];
-      if (r) {
+    for (int r = 0; r < R; r++) v[r] = src[fslot(j + r * jobs_per)];
+    if (Ns > 1) {
+#pragma unroll
+      for (int r = 1; r < R; r++) {
         float2 w = tw[r * k * step];  // r k step < L: r < R, k < Ns, step = L / (Ns R)
         if (dir > 0) w.y = -w.y;
-        x = cmul(x, w);
+        v[r] = cmul(v[r], w);
       }
-      v[r] = x;
     }
     dft_small<R>(v, dir);
     int d0 = jn * Ns * R + k;
@@ -507,29 +505,59 @@ TPM_D void stockham_stage(const float2 *in, float2 *out, const float2 *tw, int L
   }
 }
 
+struct FftArgs {
+  int n, hx, L;       // mesh size, n/2+1, pencil length of this pass
+  int nf;
+  int radix[16];
+  Div dj[16], dn[16];  // quotients by L / radix and by the product of the earlier radices
+  int P;              // pencils per block
+  Div dL, dH, dP;     // quotients by L, hx and P
+};
+
+static FftArgs fft_args(int n, int L, int P) {
+  FftArgs a;
+  a.n = n;
+  a.hx = n / 2 + 1;
+  a.L = L;
+  Factors f = factorize(L);
+  a.nf = f.nf;
+  int Ns = 1;
+  for (int i = 0; i < 16; i++) {
+    a.radix[i] = i < f.nf ? f.r[i] : 1;
+    a.dj[i] = make_div(L / a.radix[i]);
+    a.dn[i] = make_div(Ns);
+    Ns *= a.radix[i];
+  }
+  a.P = P;
+  a.dL = make_div(L);
+  a.dH = make_div(a.hx);
+  a.dP = make_div(P);
+  return a;
+}
+
 // Transforms P pencils of length L (pencil p at p * ld, element m at slot
 // fslot(m), ld >= fslots(L)) from a to scratch b
 // and back as needed; returns the buffer holding the result. dir = -1
 // forward, +1 backward (unnormalised, FFTW sign convention).
-__device__ float2 *fft_pencils(float2 *a, float2 *b, const float2 *tw, int L, int ld, int P, float dir,
-                               const int *radix, int nf) {
-  int tid = threadIdx.x, nth = blockDim.x;
+__device__ float2 *fft_pencils(float2 *a, float2 *b, const float2 *tw, int ld, int P, float dir, const FftArgs &fa) {
+  const int tid = threadIdx.x, nth = blockDim.x, L = fa.L;
   int Ns = 1;
   float2 *in = a, *out = b;
-  for (int s = 0; s < nf; s++) {
-    int R = radix[s];
+  for (int s = 0; s < fa.nf; s++) {
+    const int R = fa.radix[s];
+    const Div &dj = fa.dj[s], &dn = fa.dn[s];
     if (R == 16)
-      stockham_stage<16>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<16>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     else if (R == 8)
-      stockham_stage<8>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<8>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     else if (R == 4)
-      stockham_stage<4>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<4>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     else if (R == 2)
-      stockham_stage<2>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<2>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     else if (R == 3)
-      stockham_stage<3>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<3>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     else
-      stockham_stage<5>(in, out, tw, L, ld, Ns, P, dir, tid, nth);
+      stockham_stage<5>(in, out, tw, L, ld, Ns, P, dir, dj, dn, tid, nth);
     __syncthreads();
     Ns *= R;
     float2 *t = in;
@@ -537,25 +565,6 @@ __device__ float2 *fft_pencils(float2 *a, float2 *b, const float2 *tw, int L, in
     out = t;
   }
   return in;
-}
-
-struct FftArgs {
-  int n, hx, L;       // mesh size, n/2+1, pencil length of this pass
-  int nf;
-  int radix[16];
-  int P;              // pencils per block
-};
-
-static FftArgs fft_args(int n, int L, int P, int rmax) {
-  FftArgs a;
-  a.n = n;
-  a.hx = n / 2 + 1;
-  a.L = L;
-  Factors f = factorize(L, rmax);
-  a.nf = f.nf;
-  for (int i = 0; i < 16; i++) a.radix[i] = i < f.nf ? f.r[i] : 1;
-  a.P = P;
-  return a;
 }
 
 // twiddle table exp(-2 pi i k / L), k < L
@@ -624,7 +633,7 @@ __global__ void k_fft_x_r2c(const float *__restrict__ rho, float2 *__restrict__ 
   for (int k = tid; k < L; k += nth) twl[k] = tw_L[k];
   int64_t row0 = (int64_t)blockIdx.x * P;
   bool packed = (L * 2 == n);
-  const Div dL = make_div(L), dH = make_div(hx);
+  const Div dL = a.dL, dH = a.dH;
   for (int e0 = tid; e0 < P * L; e0 += kLoadBatch * nth) {
     float2 v[kLoadBatch];
 #pragma unroll
@@ -651,7 +660,7 @@ __global__ void k_fft_x_r2c(const float *__restrict__ rho, float2 *__restrict__ 
     }
   }
   __syncthreads();
-  float2 *res = fft_pencils(A, B, twl, L, ld, P, -1.f, a.radix, a.nf);
+  float2 *res = fft_pencils(A, B, twl, ld, P, -1.f, a);
   for (int e = tid; e < P * hx; e += nth) {
     int p = dH.q(e), k = e - p * hx;
     int64_t row = row0 + p;
@@ -766,7 +775,7 @@ __global__ void k_fft_cols(float2 *__restrict__ spec, float2 *__restrict__ spec2
   int64_t stride = axis == 1 ? (int64_t)hx : (int64_t)n * hx;
   int64_t base = axis == 1 ? (int64_t)outer * n * hx : (int64_t)outer * hx;
   int tw_ = min(TX, hx - kx0);
-  const Div dP = make_div(P), dL = make_div(L);
+  const Div dP = a.dP, dL = a.dL;
   for (int e0 = tid; e0 < P * L; e0 += kLoadBatch * nth) {
     float2 v[kLoadBatch];
 #pragma unroll
@@ -786,7 +795,7 @@ __global__ void k_fft_cols(float2 *__restrict__ spec, float2 *__restrict__ spec2
     }
   }
   __syncthreads();
-  float2 *res = fft_pencils(A, B, twl, L, Lp, P, dir, a.radix, a.nf);
+  float2 *res = fft_pencils(A, B, twl, Lp, P, dir, a);
   if (with_green && ga.pk) {
     float *sbin = reinterpret_cast<float *>(B + P * Lp);
     for (int e = tid; e < 2 * (n + 1); e += nth) sbin[e] = 0.f;
@@ -842,7 +851,7 @@ __global__ void k_fft_cols(float2 *__restrict__ spec, float2 *__restrict__ spec2
     }
     __syncthreads();
     float2 *other = res == A ? B : A;
-    res = fft_pencils(res, other, twl, L, Lp, P, 1.f, a.radix, a.nf);
+    res = fft_pencils(res, other, twl, Lp, P, 1.f, a);
   }
   for (int e = tid; e < P * L; e += nth) {
     int m = dP.q(e), q = e - m * P;
@@ -868,7 +877,7 @@ __global__ void k_fft_x_c2r(const float2 *__restrict__ spec, float *__restrict__
   int64_t row0 = (int64_t)blockIdx.x * P;
   bool packed = (L * 2 == n);
   constexpr int kB = kLoadBatch / 2;  // two loads per element
-  const Div dL = make_div(L);
+  const Div dL = a.dL;
   for (int e0 = tid; e0 < P * L; e0 += kB * nth) {
     float2 xa[kB], xb[kB];
 #pragma unroll
@@ -913,7 +922,7 @@ __global__ void k_fft_x_c2r(const float2 *__restrict__ spec, float *__restrict__
     }
   }
   __syncthreads();
-  float2 *res = fft_pencils(A, B, twl, L, ld, P, 1.f, a.radix, a.nf);
+  float2 *res = fft_pencils(A, B, twl, ld, P, 1.f, a);
   // threads run over (pencil, x) pairs of the block's rows, x in
   // [-kGhost, n + kGhost) (n >= 16 > kGhost, so one wrap maps x into [0, n))
   const int W = n + 2 * kGhost;
@@ -961,26 +970,31 @@ __global__ void k_fft_x_c2r(const float2 *__restrict__ spec, float *__restrict__
   }
 }
 
-static int pencils_for(int L, int want = 0) {
+static int pencils_for(int L, int64_t nrows, int want = 0) {
   if (want > 0) {
     // a tuned count, kept within the 160 KB of shared memory
     int cap = (int)(((160 * 1024) / (int)sizeof(float2) - L) / (2 * fslots(L)));
     return std::max(1, std::min(want, cap));
   }
-  int P = 4096 / L;
-  if (P < 1) P = 1;
-  if (P > 64) P = 64;
+  // 16 rows a block (of 16 to 320 cells a side it was the fastest or within 1%;
+  // 64 rows at 64^3, 64 blocks in all, cost 14% more), fewer where that leaves
+  // SMs without a block or the rows are long
+  int P = std::min(16, std::max(1, 4096 / L));
+  while (P > 4 && nrows < (int64_t)148 * P) P /= 2;
   return P;
 }
 
-// Columns per block of the y and z passes: 8 (16 below n = 256) consecutive
-// kx, fewer where the block's shared memory (twiddles + two buffers of
-// nspec * TX pencils) would exceed 160 KB.
+// Columns per block of the y and z passes: 16 pencils over both spectra, halved
+// while the block's shared memory (twiddles + two buffers of them) leaves room
+// for less than two blocks per SM. Two spectra at 512: 8 columns (143 KB, one
+// block) 8.2 ms, 4 columns 6.6 ms; at 128: 16 columns 152 us, 8 columns 144 us.
 static int cols_per_block(int n, int hx, int nspec, int want = 0) {
-  int TX = want > 0 ? want : (n >= 256 ? 8 : 16);
-  // room for the power-spectrum bins (2(n+1) floats) as well
-  int tmax = (int)(((160 * 1024 - 8 * (n + 1)) / (int)sizeof(float2) - n) / (2 * nspec * (fslots(n) + 15)));
-  if (TX > tmax) TX = tmax;
+  auto bytes = [&](int tx) { return (int64_t)sizeof(float2) * (n + 2 * (int64_t)nspec * tx * (fslots(n) + 15)); };
+  int TX = want;
+  if (want <= 0)
+    for (TX = 16 / nspec; TX > 1 && bytes(TX) > 110 * 1024;) TX /= 2;
+  // within 160 KB, with room for the power-spectrum bins (2(n+1) floats)
+  while (TX > 1 && bytes(TX) + 8 * (n + 1) > 160 * 1024) TX--;
   if (TX > hx) TX = hx;
   if (TX < 1) TX = 1;
   return TX;
@@ -1055,8 +1069,8 @@ void launch_poisson(const MeshGeom &g, const FftPlan &p, const float *rho, float
   int64_t nrows = (int64_t)n * n;
   bool packed = (n % 2) == 0;
   int Lx = packed ? n / 2 : n;
-  int Px = pencils_for(Lx, want_px);
-  FftArgs ax = fft_args(n, Lx, Px, kXRadixMax);
+  int Px = pencils_for(Lx, nrows, want_px);
+  FftArgs ax = fft_args(n, Lx, Px);
   const float2 *twL = packed ? p.tw_half : p.tw;
   size_t smx = sizeof(float2) * (Lx + 2 * Px * fslots(Lx));
   int thx = 256;
@@ -1065,7 +1079,7 @@ void launch_poisson(const MeshGeom &g, const FftPlan &p, const float *rho, float
   if (rho2) k_fft_x_r2c<<<(unsigned)((nrows + Px - 1) / Px), thx, smx, st>>>(rho2, spec2, ax, twL, p.tw, nrows);
   // columns
   int TX = cols_per_block(n, g.hx, nspec, want_tx);
-  FftArgs ac = fft_args(n, n, TX * nspec, kColRadixMax);
+  FftArgs ac = fft_args(n, n, TX * nspec);
   size_t smc = sizeof(float2) * (n + 2 * TX * nspec * col_stride(n, TX * nspec)) +
                (pk ? sizeof(float) * 2 * (n + 1) : 0);
   int ntx = (g.hx + TX - 1) / TX;
@@ -1096,13 +1110,13 @@ void fft_forward(const MeshGeom &g, const FftPlan &p, const float *real, float2 
   int64_t nrows = (int64_t)n * n;
   bool packed = (n % 2) == 0;
   int Lx = packed ? n / 2 : n;
-  int Px = pencils_for(Lx);
-  FftArgs ax = fft_args(n, Lx, Px, kXRadixMax);
+  int Px = pencils_for(Lx, nrows);
+  FftArgs ax = fft_args(n, Lx, Px);
   size_t smx = sizeof(float2) * (Lx + 2 * Px * fslots(Lx));
   k_fft_x_r2c<<<(unsigned)((nrows + Px - 1) / Px), 256, smx, st>>>(real, spec, ax, packed ? p.tw_half : p.tw,
                                                                    p.tw, nrows);
   int TX = cols_per_block(n, g.hx, 1);
-  FftArgs ac = fft_args(n, n, TX, kColRadixMax);
+  FftArgs ac = fft_args(n, n, TX);
   size_t smc = sizeof(float2) * (n + 2 * TX * col_stride(n, TX));
   int ntx = (g.hx + TX - 1) / TX;
   GreenArgs ga;
@@ -1116,11 +1130,11 @@ void fft_inverse(const MeshGeom &g, const FftPlan &p, float2 *spec, float *phi_p
   int64_t nrows = (int64_t)n * n;
   bool packed = (n % 2) == 0;
   int Lx = packed ? n / 2 : n;
-  int Px = pencils_for(Lx);
-  FftArgs ax = fft_args(n, Lx, Px, kXRadixMax);
+  int Px = pencils_for(Lx, nrows);
+  FftArgs ax = fft_args(n, Lx, Px);
   size_t smx = sizeof(float2) * (Lx + 2 * Px * fslots(Lx));
   int TX = cols_per_block(n, g.hx, 1);
-  FftArgs ac = fft_args(n, n, TX, kColRadixMax);
+  FftArgs ac = fft_args(n, n, TX);
   size_t smc = sizeof(float2) * (n + 2 * TX * col_stride(n, TX));
   int ntx = (g.hx + TX - 1) / TX;
   GreenArgs ga;
