@@ -1221,8 +1221,21 @@ TPM_D void fda_node_gradients(const float *boxf, float *gx, float *gy, float *gz
     // value at node coordinate i - R
     float v[kLine];
     if (axis == 0) {
+      // the row in 16-byte loads: scalar ones of lanes one row (96 bytes) apart
+      // would meet eight to a bank
+      const float4 *row = reinterpret_cast<const float4 *>(&box[q - 1 + B::H][p - 1 + B::H][0]);
+      constexpr int kAt = B::X0 - 1 - R;
+      float w[B::BX];
 #pragma unroll
-      for (int i = 0; i < kLine; i++) v[i] = box[q - 1 + B::H][p - 1 + B::H][B::X0 - 1 - R + i];
+      for (int i = kAt / 4; i <= (kAt + kLine - 1) / 4; i++) {
+        float4 t = row[i];
+        w[4 * i] = t.x;
+        w[4 * i + 1] = t.y;
+        w[4 * i + 2] = t.z;
+        w[4 * i + 3] = t.w;
+      }
+#pragma unroll
+      for (int i = 0; i < kLine; i++) v[i] = w[kAt + i];
     } else if (axis == 1) {
 #pragma unroll
       for (int i = 0; i < kLine; i++) v[i] = box[q - 1 + B::H][B::H - 1 - R + i][p - 1 + B::X0];
@@ -1230,23 +1243,30 @@ TPM_D void fda_node_gradients(const float *boxf, float *gx, float *gy, float *gz
 #pragma unroll
       for (int i = 0; i < kLine; i++) v[i] = box[B::H - 1 - R + i][q - 1 + B::H][p - 1 + B::X0];
     }
+    float f[kNodes + 1];
+    f[kNodes] = 0.f;
 #pragma unroll
     for (int a = 0; a < kNodes; a++) {
       const float *w = v + a + R;
-      float f;
       if (R == 2) {
         const float f1 = (4.f / 3.f) / 2.f, f2 = (-1.f / 3.f) / 4.f;
-        f = f1 * (w[-1] - w[1]) + f2 * (w[-2] - w[2]);
+        f[a] = f1 * (w[-1] - w[1]) + f2 * (w[-2] - w[2]);
       } else {
         const float c1 = 4.f / 5.f, c2 = -1.f / 5.f, c3 = 4.f / 105.f, c4 = -1.f / 280.f;
-        f = c1 * (w[-1] - w[1]) + c2 * (w[-2] - w[2]) + c3 * (w[-3] - w[3]) + c4 * (w[-4] - w[4]);
+        f[a] = c1 * (w[-1] - w[1]) + c2 * (w[-2] - w[2]) + c3 * (w[-3] - w[3]) + c4 * (w[-4] - w[4]);
       }
-      if (axis == 0)
-        gx[a + kGradSy * p + kGradSz * q] = f;
-      else if (axis == 1)
-        gy[p + kGradSy * a + kGradSz * q] = f;
-      else
-        gz[p + kGradSy * q + kGradSz * a] = f;
+    }
+    if (axis == 0) {
+      // the row with its spare twelfth slot
+      float4 *dst = reinterpret_cast<float4 *>(gx + kGradSy * p + kGradSz * q);
+#pragma unroll
+      for (int i = 0; i < 3; i++) dst[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+    } else if (axis == 1) {
+#pragma unroll
+      for (int a = 0; a < kNodes; a++) gy[p + kGradSy * a + kGradSz * q] = f[a];
+    } else {
+#pragma unroll
+      for (int a = 0; a < kNodes; a++) gz[p + kGradSy * q + kGradSz * a] = f[a];
     }
   }
 }
