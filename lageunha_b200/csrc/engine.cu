@@ -335,6 +335,11 @@ static void free_particles(tpm_ctx *c) {
   c->cap = 0;
 }
 
+// Words of the sort's scratch.
+static int64_t sort_words(int64_t np) {
+  return std::max(256 * (sort_tiles(np) + 1), sweep_words(std::min<int64_t>(np, (1ll << 30) - 1)));
+}
+
 static int ensure_particles(tpm_ctx *c, int64_t np) {
   if (np <= c->cap) return 0;
   CK(cudaStreamSynchronize(c->st));
@@ -352,7 +357,7 @@ static int ensure_particles(tpm_ctx *c, int64_t np) {
   CK(dmalloc(c->arena, &c->ftree, sizeof(float) * 3 * cap));
   CK(dmalloc(c->arena, &c->fout, sizeof(float) * 3 * cap));
   int64_t ntiles = sort_tiles(cap);
-  CK(dmalloc(c->arena, &c->ss.hist, sizeof(uint32_t) * 256 * (ntiles + 1)));
+  CK(dmalloc(c->arena, &c->ss.hist, sizeof(uint32_t) * sort_words(cap)));
   CK(dmalloc(c->arena, &c->ss.dtotal, sizeof(uint32_t) * 256));
   c->ss.cap_tiles = ntiles;
   // tree: every node holds >= 1 particle and every inner node >= 10, so the
@@ -517,7 +522,7 @@ int64_t tpm::ctx_bytes(int n_mesh, int64_t np) {
   int64_t mesh = 2 * (4 * n3 + 8 * g.spec_elems + 4 * (int64_t)g.px * g.py * g.pz) + 4 * g.spec_elems;
   int64_t ncubes = 1ll << (3 * (g.cbits - 2));
   mesh += 3 * 4 * (ncubes + 1) + 8 * (int64_t)(n_mesh + n_mesh / 2 + 1);
-  int64_t parts = np * (12 + 12 + 8 + 8 + 4 + 4 + 12 + 12 + 12 + 12) + 4 * 256 * (sort_tiles(np) + 1) + 1024;
+  int64_t parts = np * (12 + 12 + 8 + 8 + 4 + 4 + 12 + 12 + 12 + 12) + 4 * sort_words(np) + 1024;
   int64_t cap_nodes = np + np / 4 + 64;
   int64_t tree = cap_nodes * (3 * 16 + 32 + 16);
   tree += 4 * tree_scratch_words(np, ncubes) + 8 * (np + ncubes + 16);
@@ -752,19 +757,24 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
   CK(cudaMemsetAsync(c->err, 0, sizeof(uint32_t) * 8, st));
   if (timing) CK(cudaEventRecord(c->ev[0], st));
   // ---- sort
-  launch_make_keys(c->pos, np, (uint32_t)g.n, g.sub_bits, c->key, c->val, st);
-  uint64_t *k = c->key;
-  uint32_t *v = c->val;
-  uint64_t *kalt = c->key_alt;
-  uint32_t *valt = c->val_alt;
-  radix_sort_pairs(&k, &v, kalt, valt, np, kKeyBits, c->ss, st, &c->launches);
-  c->skey = k;
-  c->perm = v;
-  launch_gather_pos(c->pos, c->perm, np, c->spos, st);
-  // the particle ranges of the 4-cell cubes and, at every eighth entry, of the
-  // PM chain's 8-cell tiles
-  launch_range_table(c->skey, np, 3 * (g.sub_bits + 2), (uint32_t)c->tb.ncubes4, c->tb.start_cube, st);
-  c->launches += 3;
+  if (sweep_sorts(np)) {
+    c->perm = sweep_sort(c->pos, np, (uint32_t)g.n, g.sub_bits, reinterpret_cast<uint32_t *>(c->key_alt), c->val,
+                         c->val_alt, c->ss.hist, c->err, st, &c->launches);
+    c->skey = c->key;
+  } else {
+    launch_make_keys(c->pos, np, (uint32_t)g.n, g.sub_bits, c->key, c->val, st);
+    uint64_t *k = c->key;
+    uint32_t *v = c->val;
+    radix_sort_pairs(&k, &v, c->key_alt, c->val_alt, np, kKeyBits, c->ss, st, &c->launches);
+    c->skey = k;
+    c->perm = v;
+    c->launches += 1;
+  }
+  // the sorted positions and keys, and the particle ranges of the 4-cell cubes
+  // (at every eighth entry, of the PM chain's 8-cell tiles)
+  launch_gather_pos(c->pos, c->perm, np, (uint32_t)g.n, g.sub_bits, c->spos, c->skey, 3 * (g.sub_bits + 2),
+                    (uint32_t)c->tb.ncubes4, c->tb.start_cube, st);
+  c->launches += 1;
   CK(stage_check(st, "sort"));
   if (timing) CK(cudaEventRecord(c->ev[1], st));
   // ---- PM: with both parts, on st_pm beside the tree build
@@ -856,6 +866,7 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
     if (herr[0] & kErrNodeOverflow) return fail(TPM_E_OVERFLOW, "tree node capacity exceeded");
     if (herr[0] & kErrStackOverflow) return fail(TPM_E_OVERFLOW, "tree-walk stack overflow");
     if (herr[0] & kErrTmaTimeout) return fail(TPM_E_CUDA, "TMA load timed out in fda4");
+    if (herr[0] & kErrSortWait) return fail(TPM_E_CUDA, "a sort tile waited too long for its predecessor");
     return fail(TPM_E_CUDA, "device error flags 0x%x", herr[0]);
   }
   if (timing) {

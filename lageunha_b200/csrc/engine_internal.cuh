@@ -16,11 +16,12 @@ enum DeviceError : uint32_t {
   kErrNodeOverflow = 2u,     // tree node capacity exceeded
   kErrTmaTimeout = 4u,       // a TMA transaction did not complete in time
   kErrListOverflow = 8u,     // interaction list overflow
+  kErrSortWait = 16u,        // a sort tile's predecessor did not report in time
 };
 
 // ---------------------------------------------------------------- sort
 struct SortScratch {
-  uint32_t *hist = nullptr;  // [256][ntiles]
+  uint32_t *hist = nullptr;  // [256][ntiles], or the single sweep's words
   uint32_t *dtotal = nullptr;  // [256]
   int64_t cap_tiles = 0;
 };
@@ -35,8 +36,17 @@ void launch_make_keys(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits,
 void radix_sort_pairs(uint64_t **key, uint32_t **val, uint64_t *key_alt, uint32_t *val_alt,
                       int64_t np, int nbits, SortScratch &scr, cudaStream_t st, int64_t *launches);
 int64_t sort_tiles(int64_t np);
-void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, uint32_t *spos,
-                       cudaStream_t st);
+// The single-sweep sort of np particles (sweep_sorts(np): its counters hold
+// them): the permutation, in val or val_alt. key32: 2 np words, scratch:
+// sweep_words(np) words.
+bool sweep_sorts(int64_t np);
+int64_t sweep_words(int64_t np);
+uint32_t *sweep_sort(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits, uint32_t *key32, uint32_t *val,
+                     uint32_t *val_alt, uint32_t *scratch, uint32_t *err, cudaStream_t st, int64_t *launches);
+// Positions, full keys and cube ranges (launch_range_table's, of the keys >>
+// shift) of the sorted particles.
+void launch_gather_pos(const uint32_t *pos, uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
+                       uint64_t *skey, int shift, uint32_t ntable, uint32_t *start, cudaStream_t st);
 // start[t] = first sorted index whose key >> shift >= t, t in [0, ntable].
 // (A Morton cube's eight sub-cubes are consecutive, so the table of the 4-cell
 // cubes at every eighth entry is that of the 8-cell tiles.)

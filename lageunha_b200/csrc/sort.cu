@@ -8,6 +8,15 @@
 // sub-cell bits) and the (key, index) pairs are sorted by a stable LSD radix
 // sort with 8-bit digits. Ties keep the input order, so the permutation is
 // the stable argsort of the keys and is bit-exact against a CPU recomputation.
+//
+// A force evaluation sorts in single-sweep passes (sweep_sort): the digit
+// counts of all five passes come from one read of the positions, each pass
+// places its tiles by looking back at its predecessors' counts, and carries 8
+// bytes per particle: the 7 bits of the first pass are not needed again, the
+// rest of the key fits 32 bits, and the full keys of the sorted particles are
+// recomputed when their positions are gathered. radix_sort_pairs (a histogram
+// and a scan per pass, 64-bit keys) remains for callers without scratch for
+// the look-back (tpm_morton_order_noalloc) and for 2^30 particles and more.
 #include "engine_internal.cuh"
 
 namespace tpm {
@@ -247,28 +256,302 @@ void radix_sort_pairs(uint64_t **key, uint32_t **val, uint64_t *key_alt, uint32_
   *val = vin;
 }
 
-__global__ void k_gather_pos(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ perm,
-                             int64_t np, uint32_t *__restrict__ spos) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t p = perm[i];
-    spos[3 * i + 0] = pos[3 * (int64_t)p + 0];
-    spos[3 * i + 1] = pos[3 * (int64_t)p + 1];
-    spos[3 * i + 2] = pos[3 * (int64_t)p + 2];
+// ------------------------------------------------------------ single sweep
+constexpr int kSweepThreads = 512;
+constexpr int kSweepWarps = kSweepThreads / 32;
+constexpr int kSweepItems = 8;
+constexpr int kSweepTile = kSweepThreads * kSweepItems;
+constexpr int kSweepPasses = 5;
+constexpr int kLowBits = kKeyBits - 32;  // sorted by the first pass and dropped
+// words before the tile states: the digit counts of every pass and the passes'
+// tile tickets
+constexpr int kSweepHead = kSweepPasses * 256 + 8;
+// A tile's word per digit: its own count (kOwn) or that of all tiles up to and
+// with it (kAll)
+constexpr uint32_t kOwn = 1u << 30, kAll = 2u << 30, kCount = kOwn - 1u;
+
+int64_t sweep_words(int64_t np) { return kSweepHead + 256 * kSweepPasses * ((np + kSweepTile - 1) / kSweepTile); }
+
+TPM_D uint64_t key_of(const uint32_t *__restrict__ pos, int64_t i, uint32_t n, int sub_bits) {
+  return morton3(quantize(pos[3 * i + 0], n, sub_bits), quantize(pos[3 * i + 1], n, sub_bits),
+                 quantize(pos[3 * i + 2], n, sub_bits));
+}
+
+// Digit counts of all passes: counts[pass * 256 + digit].
+__global__ void __launch_bounds__(512) k_sweep_count(const uint32_t *__restrict__ pos, int64_t np, uint32_t n,
+                                                     int sub_bits, uint32_t *__restrict__ counts) {
+  __shared__ uint32_t h[4][kSweepPasses * 256];  // four copies: warps of one copy seldom meet
+  for (int i = threadIdx.x; i < 4 * kSweepPasses * 256; i += blockDim.x) (&h[0][0])[i] = 0u;
+  __syncthreads();
+  uint32_t *mine = h[(threadIdx.x >> 5) & 3];
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = key_of(pos, i, n, sub_bits);
+    atomicAdd(&mine[(uint32_t)k & ((1u << kLowBits) - 1u)], 1u);
+    const uint32_t hi = (uint32_t)(k >> kLowBits);
+#pragma unroll
+    for (int p = 1; p < kSweepPasses; p++) atomicAdd(&mine[p * 256 + ((hi >> (8 * (p - 1))) & 0xffu)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kSweepPasses * 256; i += blockDim.x) {
+    uint32_t v = h[0][i] + h[1][i] + h[2][i] + h[3][i];
+    if (v) atomicAdd(&counts[i], v);
   }
 }
 
-void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, uint32_t *spos,
-                       cudaStream_t st) {
-  int blocks = (int)((np + 255) / 256);
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  if (blocks < 1) blocks = 1;
-  k_gather_pos<<<blocks, 256, 0, st>>>(pos, perm, np, spos);
+// One pass over one tile of kSweepTile items. kFirst: the items are the
+// particles in the caller's order, the digit the key's low bits; else (key,
+// index) pairs with the digit at `shift` of the 32-bit key. kLast: the keys are
+// not written.
+//
+// Ranks: warp w owns 256 consecutive items. For each chunk of 32 the first lane
+// of every digit adds the digit's lanes to the warp's counter, and the old
+// values are read back after all chunks have issued theirs, so the chain of a
+// counter's updates runs at the shared memory's rate and not at its latency.
+// Tiles take their numbers in the order in which they start, so a tile's
+// predecessors are running or done when it looks back at them, and every wait
+// ends; it is bounded all the same (err gets kErrSortWait).
+template <bool kFirst, bool kLast>
+__global__ void __launch_bounds__(kSweepThreads, 2)
+    k_sweep_pass(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
+                 uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t np, uint32_t n, int sub_bits,
+                 int shift, const uint32_t *__restrict__ counts, uint32_t *__restrict__ ticket,
+                 uint32_t *__restrict__ state, uint32_t *__restrict__ err) {
+  extern __shared__ __align__(16) uint32_t sw_smem[];
+  uint32_t *sk = sw_smem, *sv = sk + kSweepTile;                          // the tile in digit order
+  uint32_t(*wc)[256] = reinterpret_cast<uint32_t(*)[256]>(sv + kSweepTile);  // [warps][256]
+  __shared__ uint32_t lstart[256], gbase[256], ws[8], wg[8], tile_sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) tile_sh = atomicAdd(ticket, 1u);
+  for (int i = tid; i < kSweepWarps * 256; i += kSweepThreads) (&wc[0][0])[i] = 0u;
+  __syncthreads();
+  const int64_t tile = tile_sh, tbase = tile * kSweepTile;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int64_t i0 = tbase + warp * (kSweepItems * 32) + lane;
+  uint32_t k[kSweepItems], v[kSweepItems], d[kSweepItems];
+#pragma unroll
+  for (int c = 0; c < kSweepItems; c++) {
+    const int64_t i = i0 + 32 * c;
+    const bool ok = i < np;
+    k[c] = v[c] = 0u;
+    d[c] = 0x100u;
+    if (kFirst) {
+      if (ok) {
+        const uint64_t key = key_of(pos, i, n, sub_bits);
+        k[c] = (uint32_t)(key >> kLowBits);
+        v[c] = (uint32_t)i;
+        d[c] = (uint32_t)key & ((1u << kLowBits) - 1u);
+      }
+    } else if (ok) {
+      k[c] = kin[i];
+      v[c] = vin[i];
+      d[c] = (k[c] >> shift) & 0xffu;
+    }
+  }
+  uint32_t peers[kSweepItems], old[kSweepItems];
+#pragma unroll
+  for (int c = 0; c < kSweepItems; c++) {
+    // the lanes with this lane's digit, by one vote per bit (a match
+    // instruction is slower: 197 us for the pass over 16.8 million pairs)
+    uint32_t same = __ballot_sync(0xffffffffu, d[c] < 0x100u);
+    if (d[c] >= 0x100u) same = ~same;
+#pragma unroll
+    for (int b = 0; b < (kFirst ? kLowBits : 8); b++) {
+      const bool bit = (d[c] >> b) & 1u;
+      const uint32_t with = __ballot_sync(0xffffffffu, bit);
+      same &= bit ? with : ~with;
+    }
+    peers[c] = same;
+    old[c] = 0u;
+    if (d[c] < 0x100u && (peers[c] & lt) == 0) old[c] = atomicAdd(&wc[warp][d[c]], (uint32_t)__popc(peers[c]));
+    __syncwarp();
+  }
+#pragma unroll
+  for (int c = 0; c < kSweepItems; c++)  // the rank within the warp's items of the digit
+    old[c] = __shfl_sync(0xffffffffu, old[c], __ffs(peers[c]) - 1) + (uint32_t)__popc(peers[c] & lt);
+  __syncthreads();
+  // ---- per digit: prefix over the warps, the tile's count, its place
+  if (tid < 256) {
+    uint32_t run = 0;
+#pragma unroll
+    for (int w = 0; w < kSweepWarps; w++) {
+      uint32_t t = wc[w][tid];
+      wc[w][tid] = run;
+      run += t;
+    }
+    uint32_t *mine = state + tile * 256 + tid;
+    // the count travels with its flag in one word, so no fence is needed
+    *reinterpret_cast<volatile uint32_t *>(mine) = run | (tile == 0 ? kAll : kOwn);
+    uint32_t x = run, g = counts[tid];
+    const uint32_t total = g;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      uint32_t z = __shfl_up_sync(0xffffffffu, g, o);
+      if (lane >= o) {
+        x += y;
+        g += z;
+      }
+    }
+    if (lane == 31) {
+      ws[warp] = x;
+      wg[warp] = g;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    uint32_t px = 0, pg = 0;
+    for (int w = 0; w < warp; w++) {
+      px += ws[w];
+      pg += wg[w];
+    }
+    lstart[tid] = px + x - run;
+    // look back, four tiles at a time
+    uint32_t before = 0;
+    int64_t t = tile - 1;
+    uint32_t spins = 0;
+    while (t >= 0) {
+      uint32_t s[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        s[q] = t - q >= 0 ? *reinterpret_cast<const volatile uint32_t *>(state + (t - q) * 256 + tid) : kAll;
+      bool done = false;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (done || s[q] < kOwn) break;
+        before += s[q] & kCount;
+        t--;
+        done = s[q] >= kAll;
+      }
+      if (done) break;
+      if (++spins > (1u << 22)) {
+        atomicOr(err, (uint32_t)kErrSortWait);
+        break;
+      }
+    }
+    if (tile > 0) *reinterpret_cast<volatile uint32_t *>(mine) = (before + run) | kAll;
+    gbase[tid] = pg + g - total + before;
+  }
+  __syncthreads();
+  // ---- place every item at its slot of the tile sorted by digit
+#pragma unroll
+  for (int c = 0; c < kSweepItems; c++) {
+    if (d[c] < 0x100u) {
+      const uint32_t slot = lstart[d[c]] + wc[warp][d[c]] + old[c];
+      sk[slot] = k[c];
+      sv[slot] = v[c];
+      if (kFirst) reinterpret_cast<uint8_t *>(wc + kSweepWarps)[slot] = (uint8_t)d[c];
+    }
+  }
+  __syncthreads();
+  // ---- write out: consecutive slots of a digit go to consecutive addresses
+  const int nt = (int)(np - tbase < kSweepTile ? np - tbase : kSweepTile);
+#pragma unroll
+  for (int c = 0; c < kSweepItems; c++) {
+    const int j = tid + c * kSweepThreads;
+    if (j < nt) {
+      const uint32_t kk = sk[j];
+      const uint32_t dd = kFirst ? reinterpret_cast<uint8_t *>(wc + kSweepWarps)[j] : (kk >> shift) & 0xffu;
+      const uint32_t g = gbase[dd] + ((uint32_t)j - lstart[dd]);
+      if (!kLast) kout[g] = kk;
+      vout[g] = sv[j];
+    }
+  }
 }
 
-// Thread i writes the entries (key[i - 1] >> shift, key[i] >> shift]. Where the
-// mesh is no power of two or particles are sparse, runs of empty entries are
-// long (thousands); those are written by the whole warp.
+constexpr size_t kSweepSmem = sizeof(uint32_t) * (2 * kSweepTile + kSweepWarps * 256);
+constexpr size_t kSweepSmemFirst = kSweepSmem + kSweepTile;
+
+bool sweep_sorts(int64_t np) { return np < (int64_t)kOwn; }
+
+uint32_t *sweep_sort(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits, uint32_t *key32, uint32_t *val,
+                     uint32_t *val_alt, uint32_t *scratch, uint32_t *err, cudaStream_t st, int64_t *launches) {
+  const int64_t ntiles = (np + kSweepTile - 1) / kSweepTile;
+  uint32_t *counts = scratch, *tickets = scratch + kSweepPasses * 256, *state = scratch + kSweepHead;
+  uint32_t *ka = key32, *kb = key32 + np;
+  // an attribute of the function on the current device: set on every call, so
+  // contexts and threads on any device get it
+  cudaFuncSetAttribute(k_sweep_pass<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmemFirst);
+  cudaFuncSetAttribute(k_sweep_pass<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
+  cudaFuncSetAttribute(k_sweep_pass<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem);
+  cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * sweep_words(np), st);
+  int blocks = (int)((np + 2047) / 2048);
+  if (blocks > 148 * 4) blocks = 148 * 4;
+  k_sweep_count<<<blocks, 512, 0, st>>>(pos, np, n, sub_bits, counts);
+  k_sweep_pass<true, false><<<(unsigned)ntiles, kSweepThreads, kSweepSmemFirst, st>>>(
+      pos, nullptr, nullptr, ka, val, np, n, sub_bits, 0, counts, tickets, state, err);
+  uint32_t *vi = val, *vo = val_alt;
+  for (int p = 1; p < kSweepPasses; p++) {
+    uint32_t *stp = state + (int64_t)p * 256 * ntiles;
+    if (p < kSweepPasses - 1)
+      k_sweep_pass<false, false><<<(unsigned)ntiles, kSweepThreads, kSweepSmem, st>>>(
+          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp, err);
+    else
+      k_sweep_pass<false, true><<<(unsigned)ntiles, kSweepThreads, kSweepSmem, st>>>(
+          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp, err);
+    uint32_t *t = ka;
+    ka = kb;
+    kb = t;
+    t = vi;
+    vi = vo;
+    vo = t;
+  }
+  if (launches) *launches += 1 + kSweepPasses;
+  return vi;
+}
+
+// The entries (cube of sorted particle i - 1, cube of i] of the range table of
+// the 4-cell cubes start at i. Where the mesh is no power of two or particles
+// are sparse, runs of empty entries are long (thousands): those are written by
+// the whole warp. Called by whole warps; t < tp where there is nothing to
+// write.
+TPM_D void range_entries(int64_t tp, int64_t t, int64_t i, uint32_t *__restrict__ start) {
+  const int lane = threadIdx.x & 31;
+  const bool longrun = t - tp > 8;
+  if (!longrun)
+    for (int64_t q = tp + 1; q <= t; q++) start[q] = (uint32_t)i;
+  unsigned m = __ballot_sync(0xffffffffu, longrun);
+  while (m) {
+    const int src = __ffs(m) - 1;
+    m &= m - 1;
+    const int64_t a = __shfl_sync(0xffffffffu, tp, src), b = __shfl_sync(0xffffffffu, t, src);
+    for (int64_t q = a + 1 + lane; q <= b; q += 32) start[q] = (uint32_t)(i - lane + src);
+  }
+}
+
+// The sorted particles: their positions, full keys and the range table of the
+// cubes key >> shift (ntable of them).
+__global__ void __launch_bounds__(256) k_gather_pos(const uint32_t *__restrict__ pos, uint32_t *__restrict__ perm,
+                                                    int64_t np, uint32_t n, int sub_bits, uint32_t *__restrict__ spos,
+                                                    uint64_t *__restrict__ skey, int shift, uint32_t ntable,
+                                                    uint32_t *__restrict__ start) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); i0 <= np;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + lane;
+    uint64_t k = (uint64_t)ntable << shift;
+    if (i < np) {
+      int64_t p = perm[i];
+      if (p >= np) perm[i] = (uint32_t)(p = 0);  // only after a sort that gave up (kErrSortWait)
+      const uint32_t u[3] = {pos[3 * p + 0], pos[3 * p + 1], pos[3 * p + 2]};
+      k = key_of(u, 0, n, sub_bits);
+      spos[3 * i + 0] = u[0];
+      spos[3 * i + 1] = u[1];
+      spos[3 * i + 2] = u[2];
+      skey[i] = k;
+    }
+    int64_t t = (int64_t)(k >> shift);
+    int64_t tp = __shfl_up_sync(0xffffffffu, t, 1);
+    if (lane == 0) tp = i > 0 && i <= np ? (int64_t)(key_of(pos, min((int64_t)perm[i - 1], np - 1), n, sub_bits) >> shift) : -1;
+    if (i > np) t = tp;
+    range_entries(tp, t, i, start);
+  }
+}
+
+void launch_gather_pos(const uint32_t *pos, uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
+                       uint64_t *skey, int shift, uint32_t ntable, uint32_t *start, cudaStream_t st) {
+  int blocks = (int)((np + 256) / 256);
+  if (blocks > 148 * 32) blocks = 148 * 32;
+  k_gather_pos<<<blocks, 256, 0, st>>>(pos, perm, np, n, sub_bits, spos, skey, shift, ntable, start);
+}
+
 __global__ void k_range_table(const uint64_t *__restrict__ key, int64_t np, int shift,
                               uint32_t ntable, uint32_t *__restrict__ start) {
   const int lane = threadIdx.x & 31;
@@ -279,18 +562,8 @@ __global__ void k_range_table(const uint64_t *__restrict__ key, int64_t np, int 
     if (i <= np) {
       t = i < np ? (int64_t)(key[i] >> shift) : (int64_t)ntable;
       tp = i > 0 ? (int64_t)(key[i - 1] >> shift) : -1;
-      if (t > (int64_t)ntable) t = ntable;
     }
-    const bool longrun = t - tp > 8;
-    if (!longrun)
-      for (int64_t q = tp + 1; q <= t; q++) start[q] = (uint32_t)i;
-    unsigned m = __ballot_sync(0xffffffffu, longrun);
-    while (m) {
-      const int src = __ffs(m) - 1;
-      m &= m - 1;
-      const int64_t a = __shfl_sync(0xffffffffu, tp, src), b = __shfl_sync(0xffffffffu, t, src);
-      for (int64_t q = a + 1 + lane; q <= b; q += 32) start[q] = (uint32_t)(i0 + src);
-    }
+    range_entries(tp, t, i, start);
   }
 }
 
