@@ -272,9 +272,36 @@ constexpr uint32_t kOwn = 1u << 30, kAll = 2u << 30, kCount = kOwn - 1u;
 
 int64_t sweep_words(int64_t np) { return kSweepHead + 256 * kSweepPasses * ((np + kSweepTile - 1) / kSweepTile); }
 
+// Bits 0-9 of v at every third bit.
+TPM_D uint32_t spread10(uint32_t v) {
+  v &= 0x3ffu;
+  v = (v | (v << 16)) & 0x030000ffu;
+  v = (v | (v << 8)) & 0x0300f00fu;
+  v = (v | (v << 4)) & 0x030c30c3u;
+  return (v | (v << 2)) & 0x09249249u;
+}
+
+// Bits 10-12 of v at every third bit.
+TPM_D uint32_t spread_top(uint32_t v) {
+  v >>= 10;
+  return (v | (v << 2) | (v << 4)) & 0x49u;
+}
+
+// morton3 of the particle's quantised coordinates in 32-bit halves: the low 30
+// bits and the 9 above them.
+TPM_D void key_halves(const uint32_t *__restrict__ pos, int64_t i, uint32_t n, int sub_bits, uint32_t &lo,
+                      uint32_t &hi) {
+  static_assert(kAxisBits == 13, "10 low and 3 high bits per axis");
+  const uint32_t x = quantize(pos[3 * i + 0], n, sub_bits), y = quantize(pos[3 * i + 1], n, sub_bits),
+                 z = quantize(pos[3 * i + 2], n, sub_bits);
+  lo = spread10(x) | (spread10(y) << 1) | (spread10(z) << 2);
+  hi = spread_top(x) | (spread_top(y) << 1) | (spread_top(z) << 2);
+}
+
 TPM_D uint64_t key_of(const uint32_t *__restrict__ pos, int64_t i, uint32_t n, int sub_bits) {
-  return morton3(quantize(pos[3 * i + 0], n, sub_bits), quantize(pos[3 * i + 1], n, sub_bits),
-                 quantize(pos[3 * i + 2], n, sub_bits));
+  uint32_t lo, hi;
+  key_halves(pos, i, n, sub_bits, lo, hi);
+  return (uint64_t)hi << 30 | lo;
 }
 
 // Digit counts of all passes: counts[pass * 256 + digit].
@@ -285,9 +312,10 @@ __global__ void __launch_bounds__(512) k_sweep_count(const uint32_t *__restrict_
   __syncthreads();
   uint32_t *mine = h[(threadIdx.x >> 5) & 3];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = key_of(pos, i, n, sub_bits);
-    atomicAdd(&mine[(uint32_t)k & ((1u << kLowBits) - 1u)], 1u);
-    const uint32_t hi = (uint32_t)(k >> kLowBits);
+    uint32_t lo, hi;
+    key_halves(pos, i, n, sub_bits, lo, hi);
+    atomicAdd(&mine[lo & ((1u << kLowBits) - 1u)], 1u);
+    hi = hi << (30 - kLowBits) | lo >> kLowBits;
 #pragma unroll
     for (int p = 1; p < kSweepPasses; p++) atomicAdd(&mine[p * 256 + ((hi >> (8 * (p - 1))) & 0xffu)], 1u);
   }
@@ -327,47 +355,54 @@ __global__ void __launch_bounds__(kSweepThreads, 2)
   const int64_t tile = tile_sh, tbase = tile * kSweepTile;
   const uint32_t lt = (1u << lane) - 1u;
   const int64_t i0 = tbase + warp * (kSweepItems * 32) + lane;
-  uint32_t k[kSweepItems], v[kSweepItems], d[kSweepItems];
+  // who: this lane's digit << 16 (kNoItem past the last particle), the first
+  // lane of the digit << 8 and this lane's rank among its lanes; later the
+  // digit and the rank within the warp's items of it
+  constexpr uint32_t kNoItem = 0x100u;
+  uint32_t k[kSweepItems], v[kSweepItems], who[kSweepItems], old[kSweepItems];
 #pragma unroll
   for (int c = 0; c < kSweepItems; c++) {
     const int64_t i = i0 + 32 * c;
     const bool ok = i < np;
     k[c] = v[c] = 0u;
-    d[c] = 0x100u;
+    who[c] = kNoItem;
     if (kFirst) {
       if (ok) {
-        const uint64_t key = key_of(pos, i, n, sub_bits);
-        k[c] = (uint32_t)(key >> kLowBits);
+        uint32_t lo, hi;
+        key_halves(pos, i, n, sub_bits, lo, hi);
+        k[c] = hi << (30 - kLowBits) | lo >> kLowBits;
         v[c] = (uint32_t)i;
-        d[c] = (uint32_t)key & ((1u << kLowBits) - 1u);
+        who[c] = lo & ((1u << kLowBits) - 1u);
       }
     } else if (ok) {
       k[c] = kin[i];
       v[c] = vin[i];
-      d[c] = (k[c] >> shift) & 0xffu;
+      who[c] = (k[c] >> shift) & 0xffu;
     }
   }
-  uint32_t peers[kSweepItems], old[kSweepItems];
 #pragma unroll
   for (int c = 0; c < kSweepItems; c++) {
     // the lanes with this lane's digit, by one vote per bit (a match
     // instruction is slower: 197 us for the pass over 16.8 million pairs)
-    uint32_t same = __ballot_sync(0xffffffffu, d[c] < 0x100u);
-    if (d[c] >= 0x100u) same = ~same;
+    const uint32_t d = who[c];
+    uint32_t same = __ballot_sync(0xffffffffu, d != kNoItem);
+    if (d == kNoItem) same = ~same;
 #pragma unroll
     for (int b = 0; b < (kFirst ? kLowBits : 8); b++) {
-      const bool bit = (d[c] >> b) & 1u;
+      const bool bit = (d >> b) & 1u;
       const uint32_t with = __ballot_sync(0xffffffffu, bit);
       same &= bit ? with : ~with;
     }
-    peers[c] = same;
+    who[c] = d << 16 | (uint32_t)(__ffs(same) - 1) << 8 | (uint32_t)__popc(same & lt);
     old[c] = 0u;
-    if (d[c] < 0x100u && (peers[c] & lt) == 0) old[c] = atomicAdd(&wc[warp][d[c]], (uint32_t)__popc(peers[c]));
+    if (d != kNoItem && (same & lt) == 0) old[c] = atomicAdd(&wc[warp][d], (uint32_t)__popc(same));
     __syncwarp();
   }
 #pragma unroll
-  for (int c = 0; c < kSweepItems; c++)  // the rank within the warp's items of the digit
-    old[c] = __shfl_sync(0xffffffffu, old[c], __ffs(peers[c]) - 1) + (uint32_t)__popc(peers[c] & lt);
+  for (int c = 0; c < kSweepItems; c++) {
+    const uint32_t at = __shfl_sync(0xffffffffu, old[c], (int)(who[c] >> 8) & 31);
+    who[c] = (who[c] & 0xffff0000u) | (at + (who[c] & 0xffu));
+  }
   __syncthreads();
   // ---- per digit: prefix over the warps, the tile's count, its place
   if (tid < 256) {
@@ -433,11 +468,12 @@ __global__ void __launch_bounds__(kSweepThreads, 2)
   // ---- place every item at its slot of the tile sorted by digit
 #pragma unroll
   for (int c = 0; c < kSweepItems; c++) {
-    if (d[c] < 0x100u) {
-      const uint32_t slot = lstart[d[c]] + wc[warp][d[c]] + old[c];
+    const uint32_t d = who[c] >> 16;
+    if (d != kNoItem) {
+      const uint32_t slot = lstart[d] + wc[warp][d] + (who[c] & 0xffffu);
       sk[slot] = k[c];
       sv[slot] = v[c];
-      if (kFirst) reinterpret_cast<uint8_t *>(wc + kSweepWarps)[slot] = (uint8_t)d[c];
+      if (kFirst) reinterpret_cast<uint8_t *>(wc + kSweepWarps)[slot] = (uint8_t)d;
     }
   }
   __syncthreads();
