@@ -52,10 +52,17 @@ int tpm_power_spectrum(tpm_ctx *c, double boxsize, double *pk, double *cor, int3
     std += tpk[i] * i * i * pow(sin(thk) - thk * cos(thk), 2.0) / pow(thk, 6.0);
   }
   std = sqrt(4 * M_PI * std * 9.0);
-  // xi(r) at r = i cells by the sine transform (Correlation.c:96-102)
+  // xi(r) at r = i cells by the sine transform (Correlation.c:96-102), with the
+  // nx distinct sines sin(2 pi (i k mod nx) / nx) of its nx^2 terms
+  std::vector<double> sn(nx);
+  for (int m = 0; m < nx; m++) sn[m] = sin(2 * M_PI * m / rng);
   for (int i = 1; i < nx + 1; i++) {
-    double seper = 2 * M_PI * i / rng;
-    for (int k = 1; k < nx + 1; k++) tcor[i] += sin(k * seper) * k * tpk[k];
+    int m = 0;
+    for (int k = 1; k < nx + 1; k++) {
+      m += i;
+      m -= m >= nx ? nx : 0;
+      tcor[i] += sn[m] * k * tpk[k];
+    }
     tcor[i] = (rng + rng) * tcor[i] / i;
   }
   double corn1 = 0;
