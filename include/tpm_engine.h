@@ -392,7 +392,8 @@ int tpm_ewald(tpm_ctx *ctx, int64_t nt, const int64_t *targets, double *out);
  * number of stages written (<= n). */
 int tpm_stage_times(tpm_ctx *ctx, float *ms, int n);
 
-/* Counters of the last force evaluation: [0] tree nodes, [1] particle-
+/* Counters of the last force evaluation: [0] tree nodes (0 where the direct
+ * summation took every cube and no tree was needed), [1] particle-
  * particle interactions, [2] particle-node interactions, [3] walk groups,
  * [4] walk iterations, [5] nodes examined by the walk, [6] deepest walk stack. */
 int tpm_counters(tpm_ctx *ctx, int64_t *out, int n);

@@ -27,6 +27,10 @@ struct CapturedGraph {
   int64_t np = -1;
 };
 
+// The device status words of a context, cleared at the start of an evaluation
+// and read back in one copy: errors, TreeCounter words, level ranges.
+constexpr int kCountersAt = 8, kLevelsAt = 24, kStatusWords = kLevelsAt + 2 * (kAxisBits + 2);
+
 // Per-box evolution factors as the step graph reads them:
 // [0] fact1 (drag), [1] fact2 (kicks), [2] pfact (drift), [3] unused.
 constexpr int kFacWords = 4;
@@ -92,7 +96,7 @@ struct tpm_ctx {
   int law_n = -1;
   float law_eps = -1, law_rs = -1, law_rsphere = -1;
   int law_kind = -1;
-  uint32_t *err = nullptr;
+  uint32_t *err = nullptr;  // device status words: errors, then tb.counters and tb.level_range
   // power spectrum of the mass assignment (tpm_set_power_spectrum)
   bool measure_pk = false;
   double *pk_acc = nullptr;  // device [2][n+1]
@@ -104,7 +108,7 @@ struct tpm_ctx {
   // captured launch; herr/hfac are pinned host words the graphs copy through
   uint64_t gen = 1;
   tpm::CapturedGraph graphs[tpm::kNGraphs];
-  uint32_t *herr = nullptr;  // pinned [8]
+  uint32_t *herr = nullptr;  // pinned copy of the status words
   double *hfac = nullptr;    // pinned [kFacWords]
   double *dfac = nullptr;    // device [kFacWords]
   // where the device buffers come from: the request loop's arena, or
@@ -134,8 +138,9 @@ const std::string &last_error_string();
 // Enqueues one force evaluation of the loaded particles on st (no host
 // synchronisation); with timing, records the stage events. walk == false
 // stops before the tree walk (the tree and the groups are built): an
-// ensemble walks all its boxes in one launch.
-int enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk = true);
+// ensemble walks all its boxes in one launch. The tree is built where the
+// direct summation leaves groups to the walk, or always with whole_tree.
+int enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk = true, bool whole_tree = false);
 // The walk record of the context's current buffers.
 WalkBox ctx_walk_box(const tpm_ctx *c);
 // After the stream has finished an evaluation: checks the device error words

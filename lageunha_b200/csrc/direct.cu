@@ -48,7 +48,7 @@ constexpr int kDirRow = kDirList + 8;
 constexpr uint32_t kDirCandidates = 3500;
 constexpr float kDirFar = -1.0e4f;  // a (negated) coordinate outside every cut
 
-struct DirWarp {
+struct alignas(16) DirWarp {
   float seg[3][kDirSeg];   // the warp's share of the sources in reach, negated
   float list[3][kDirRow];  // those in reach of the current sub-group
   WalkBox box;             // the box of the current unit
@@ -60,16 +60,6 @@ struct DirTeam {
   float4 sbox[kDirTargets / kDirSub][2];   // sub-group boxes: centre, half sizes
   uint32_t next[2];                        // the team's coming unit
 };
-
-// Every third bit of c, from bit 0 (c < 2^30).
-TPM_D uint32_t compact3(uint32_t c) {
-  c &= 0x09249249u;
-  c = (c ^ (c >> 2)) & 0x030c30c3u;
-  c = (c ^ (c >> 4)) & 0x0300f00fu;
-  c = (c ^ (c >> 8)) & 0x030000ffu;
-  c = (c ^ (c >> 16)) & 0x000003ffu;
-  return c;
-}
 
 TPM_D void team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kDirTeamThreads) : "memory"); }
 
@@ -176,9 +166,7 @@ __global__ void __launch_bounds__(kDirThreads, 1)
       const uint64_t pr = (uint64_t)ur * (uint64_t)n;  // the target in cells, 32.32
       const float h = 0.5f * (float)w;
       const float off = (float)((int)(pr >> 32) - c0) + (float)(uint32_t)pr * 2.3283064365386963e-10f;
-      // cubes that only touch the reach (rsphere a multiple of four) hold no
-      // particle inside it: cube faces are whole cells, exact here
-      const float reach = rsphere * 0.999999f;
+      const float reach = rsphere * kCubeReach;
       int run[4];
       axis_runs((float)c0 - reach, (float)(c0 + w) + reach, n, run);
 #pragma unroll
@@ -218,12 +206,9 @@ __global__ void __launch_bounds__(kDirThreads, 1)
 #pragma unroll
       for (int a = 0; a < 3; a++) {
         // the second run starts at cube 0
-        int c4 = jj[a] < nrun[a] ? run0[a] + jj[a] : jj[a] - nrun[a];
+        const int c4 = jj[a] < nrun[a] ? run0[a] + jj[a] : jj[a] - nrun[a];
         cc[a] = (uint32_t)c4;
-        float lo = (float)(4 * c4), hi = (float)min(4 * c4 + 4, n);
-        float d = 0.5f * (lo + hi) - mid[a];
-        d -= (float)n * rintf(d * inv_n);
-        float e = fmaxf(fabsf(d) - 0.5f * (hi - lo) - hw[a], 0.f);
+        const float e = cube_gap(c4, mid[a], hw[a], n, inv_n);
         d2 += e * e;
       }
       if (d2 < rs2) {
@@ -232,30 +217,7 @@ __global__ void __launch_bounds__(kDirThreads, 1)
         c = dw.box.start_cube[cid + 1] - s0;
       }
     };
-    uint32_t s0, c, total = 0;
-    for (int jb = 0; jb < stotal; jb += 32) {
-      cube_range(jb + lane, s0, c);
-      total += __reduce_add_sync(0xffffffffu, min(c, 1u << 24));
-      if (total > kDirCandidates) break;
-    }
-    if (total > kDirCandidates) {
-      // left to the tree walk (every warp of the team finds the same total)
-      if (tw == 0) {
-        const uint32_t gm = (uint32_t)dw.box.group_max, ng = ((uint32_t)cnt + gm - 1) / gm;
-        uint32_t g0 = 0;
-        if (lane == 0) g0 = atomicAdd(&dw.box.counters[kCntGroups], ng);
-        g0 = __shfl_sync(0xffffffffu, g0, 0);
-        for (uint32_t g = lane; g < ng; g += 32) {
-          dw.box.groups[2 * (int64_t)(g0 + g)] = s + g * gm;
-          dw.box.groups[2 * (int64_t)(g0 + g) + 1] = min(gm, (uint32_t)cnt - g * gm);
-        }
-      }
-      if (ttid == 0) T.next[par ^ 1] = atomicAdd(unext, 1u);
-      team_sync(team);
-      par ^= 1;
-      u = T.next[par];
-      continue;
-    }
+    uint32_t s0, c;
     for (int t0 = 0; t0 < cnt; t0 += kDirTargets) {
       const int tc = min(cnt - t0, kDirTargets);
       const int nsub = (tc + kDirSub - 1) / kDirSub, per = (tc + nsub - 1) / nsub;
@@ -295,7 +257,7 @@ __global__ void __launch_bounds__(kDirThreads, 1)
       for (int jb = 0; jb < stotal; jb += 32) {
         // the batch's particles as one range of flat indices; this warp takes
         // every fourth chunk of 32
-        if (stotal > 32 || t0 > 0) cube_range(jb + lane, s0, c);
+        cube_range(jb + lane, s0, c);
         uint32_t incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -431,26 +393,74 @@ __global__ void __launch_bounds__(kDirThreads, 1)
   }
 }
 
-// The non-empty 4-cell cubes, in about their Morton order.
-__global__ void k_tree_units(const uint32_t *__restrict__ start_cube, int64_t ncubes, uint32_t *__restrict__ units,
-                             uint32_t *__restrict__ count) {
+// Every non-empty 4-cell cube, in about Morton order, to the direct summation
+// (units) or, with more than kDirCandidates particles in the cubes in reach, to
+// the tree walk as groups of at most group_max particles.
+__global__ void __launch_bounds__(256) k_tree_units(const uint32_t *__restrict__ start_cube, int64_t ncubes, int n,
+                                                    float rsphere, uint32_t group_max, uint32_t *__restrict__ units,
+                                                    uint32_t *__restrict__ groups, uint32_t *__restrict__ counters) {
   const int lane = threadIdx.x & 31;
+  const float rs2 = rsphere * rsphere, inv_n = __frcp_rn((float)n), reach = rsphere * kCubeReach;
   for (int64_t c0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); c0 < ncubes;
        c0 += (int64_t)gridDim.x * blockDim.x) {
-    int64_t c = c0 + lane;
-    bool on = c < ncubes && start_cube[c + 1] > start_cube[c];
-    unsigned m = __ballot_sync(0xffffffffu, on);
-    if (!m) continue;
-    uint32_t at = 0;
-    if (lane == 0) at = atomicAdd(count, (uint32_t)__popc(m));
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (on) units[at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)c;
+    const int64_t c = c0 + lane;
+    uint32_t s = 0, cnt = 0, total = 0;
+    if (c < ncubes) {
+      s = start_cube[c];
+      cnt = start_cube[c + 1] - s;
+    }
+    if (cnt) {
+      int run[3][4];
+      float mid[3], hw[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const int x = 4 * (int)compact3((uint32_t)c >> a), w = min(4, n - x);
+        hw[a] = 0.5f * (float)w;
+        mid[a] = (float)x + hw[a];
+        axis_runs((float)x - reach, (float)(x + w) + reach, n, run[a]);
+      }
+      auto at = [&](int a, int j) { return j < run[a][1] ? run[a][0] + j : j - run[a][1]; };  // the second run starts at 0
+      for (int jz = 0; jz < run[2][1] + run[2][3] && total <= kDirCandidates; jz++) {
+        const int cz = at(2, jz);
+        const float ez = cube_gap(cz, mid[2], hw[2], n, inv_n);
+        for (int jy = 0; jy < run[1][1] + run[1][3]; jy++) {
+          const int cy = at(1, jy);
+          const float ey = cube_gap(cy, mid[1], hw[1], n, inv_n);
+          for (int jx = 0; jx < run[0][1] + run[0][3]; jx++) {
+            const int cx = at(0, jx);
+            const float ex = cube_gap(cx, mid[0], hw[0], n, inv_n);
+            if (ex * ex + ey * ey + ez * ez < rs2) {
+              const int64_t id = (int64_t)morton3((uint32_t)cx, (uint32_t)cy, (uint32_t)cz);
+              total += min(start_cube[id + 1] - start_cube[id], 1u << 24);
+            }
+          }
+        }
+      }
+    }
+    const bool dense = total > kDirCandidates;
+    const unsigned m = __ballot_sync(0xffffffffu, cnt && !dense);
+    if (m) {
+      uint32_t first = 0;
+      if (lane == 0) first = atomicAdd(&counters[kCntUnits], (uint32_t)__popc(m));
+      first = __shfl_sync(0xffffffffu, first, 0);
+      if (cnt && !dense) units[first + __popc(m & ((1u << lane) - 1u))] = (uint32_t)c;
+    }
+    if (cnt && dense) {
+      const uint32_t ng = (cnt + group_max - 1) / group_max;
+      const int64_t g0 = atomicAdd(&counters[kCntGroups], ng);
+      for (uint32_t g = 0; g < ng; g++) {
+        groups[2 * (g0 + g)] = s + g * group_max;
+        groups[2 * (g0 + g) + 1] = min(group_max, cnt - g * group_max);
+      }
+    }
   }
 }
 
-void tree_units(TreeBuffers &tb, cudaStream_t st, int64_t *launches) {
+void tree_units(const TreeParams &tp, TreeBuffers &tb, cudaStream_t st, int64_t *launches) {
   int blocks = (int)std::min<int64_t>((tb.ncubes4 + 255) / 256, 148 * 16);
-  k_tree_units<<<blocks, 256, 0, st>>>(tb.start_cube, tb.ncubes4, tb.units, &tb.counters[kCntUnits]);
+  k_tree_units<<<blocks, 256, 0, st>>>(tb.start_cube, tb.ncubes4, (int)tp.n, tp.rsphere,
+                                       (uint32_t)std::max(1, std::min(32, tp.group_max)), tb.units, tb.groups,
+                                       tb.counters);
   if (launches) *launches += 1;
 }
 

@@ -598,27 +598,27 @@ int tpm::create_ctx(const tpm_params *params, int device, DeviceArena *arena, tp
     }
   }
   // the allocations below are mirrored by ctx_bytes()
-  if (dmalloc(c->arena, &c->err, sizeof(uint32_t) * 8) != cudaSuccess ||
-      dmalloc(c->arena, &c->tb.counters, sizeof(uint32_t) * 16) != cudaSuccess ||
-      dmalloc(c->arena, &c->tb.level_range, sizeof(uint32_t) * 2 * (kAxisBits + 2)) != cudaSuccess ||
+  if (dmalloc(c->arena, &c->err, sizeof(uint32_t) * kStatusWords) != cudaSuccess ||
       dmalloc(c->arena, &c->tb.walkbox, sizeof(WalkBox)) != cudaSuccess) {
     tpm_destroy(c);
     return fail(TPM_E_NOMEM, "cudaMalloc of context scratch failed");
   }
+  c->tb.counters = c->err + kCountersAt;
+  c->tb.level_range = c->err + kLevelsAt;
   c->tb.stack_words = walk_stack_words();
   if (dmalloc(c->arena, &c->tb.stack, sizeof(uint32_t) * c->tb.stack_words) != cudaSuccess) {
     tpm_destroy(c);
     return fail(TPM_E_NOMEM, "cudaMalloc of walk stacks failed");
   }
-  if (cudaMallocHost(&c->herr, sizeof(uint32_t) * 8) != cudaSuccess ||
+  if (cudaMallocHost(&c->herr, sizeof(uint32_t) * kStatusWords) != cudaSuccess ||
       cudaMallocHost(&c->hfac, sizeof(double) * kFacWords) != cudaSuccess ||
       dmalloc(c->arena, &c->dfac, sizeof(double) * kFacWords) != cudaSuccess) {
     tpm_destroy(c);
     return fail(TPM_E_NOMEM, "allocation of step scratch failed");
   }
-  memset(c->herr, 0, sizeof(uint32_t) * 8);
+  memset(c->herr, 0, sizeof(uint32_t) * kStatusWords);
   memset(c->hfac, 0, sizeof(double) * kFacWords);
-  cudaMemsetAsync(c->err, 0, sizeof(uint32_t) * 8, c->st);
+  cudaMemsetAsync(c->err, 0, sizeof(uint32_t) * kStatusWords, c->st);
   rc = alloc_mesh(c);
   if (!rc) rc = ensure_mesh2(c);
   if (!rc) rc = build_law(c);
@@ -644,8 +644,6 @@ int tpm_destroy(tpm_ctx *c) {
   dfree(c->arena, c->law.tlog);
   dfree(c->arena, c->law.tpc);
   dfree(c->arena, c->err);
-  dfree(c->arena, c->tb.counters);
-  dfree(c->arena, c->tb.level_range);
   dfree(c->arena, c->tb.walkbox);
   dfree(c->arena, c->tb.stack);
   dfree(c->arena, c->stage);
@@ -750,11 +748,11 @@ int tpm_load_lagrangian(tpm_ctx *c, int64_t np, const void *particles, int64_t s
 
 }  // extern "C"
 
-int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk) {
+int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk, bool whole_tree) {
   const MeshGeom &g = c->g;
   int64_t np = c->np;
   c->launches = 0;
-  CK(cudaMemsetAsync(c->err, 0, sizeof(uint32_t) * 8, st));
+  CK(cudaMemsetAsync(c->err, 0, sizeof(uint32_t) * kStatusWords, st));
   if (timing) CK(cudaEventRecord(c->ev[0], st));
   // ---- sort
   if (sweep_sorts(np)) {
@@ -830,9 +828,10 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
     tp.mass = c->prm.particle_mass;
     tp.group_max = c->tune_group_max;
     tp.group_level = c->tune_group_level;
-    tree_build(tp, c->skey, c->spos, np, c->tb, c->err, st, &c->launches);
-    CK(cudaMemsetAsync(c->tb.counters, 0, sizeof(uint32_t) * 16, st));
+    // the tree is needed for the groups that the direct summation leaves
     tree_targets(tp, c->skey, np, c->tb, c->cube_start, st, &c->launches);
+    tree_build(tp, c->skey, c->spos, np, c->tb, whole_tree ? nullptr : &c->tb.counters[kCntGroups], c->err, st,
+               &c->launches);
     CK(stage_check(st, "tree_build"));
     // the walk takes every SM: it starts once the PM chain is done too (the
     // tree_build stage of an overlapped evaluation ends with both chains)
@@ -854,11 +853,10 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
 }
 
 int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) {
-  uint32_t herr[8];
-  if (from_host) {
-    memcpy(herr, c->herr, sizeof(herr));
-  } else {
-    CK(cudaMemcpyAsync(herr, c->err, sizeof(herr), cudaMemcpyDeviceToHost, c->st));
+  // error words, counters and level ranges in one copy
+  const uint32_t *herr = c->herr;
+  if (!from_host) {
+    CK(cudaMemcpyAsync(c->herr, c->err, sizeof(uint32_t) * kStatusWords, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
   if (herr[0]) {
@@ -877,11 +875,7 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
       cudaEventElapsedTime(&ms, c->ev[s0], c->ev[s + 1]);
       c->stage_ms[s] = ms;
     }
-    // counters: nodes, pp, pc, groups
-    uint32_t hc[16];
-    uint32_t lr[2 * (kAxisBits + 2)];
-    CK(cudaMemcpy(hc, c->tb.counters, sizeof(hc), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(lr, c->tb.level_range, sizeof(lr), cudaMemcpyDeviceToHost));
+    const uint32_t *hc = herr + kCountersAt, *lr = herr + kLevelsAt;
     uint32_t nn = 0;
     for (int l = 0; l <= kAxisBits; l++)
       if (lr[2 * l + 1] > nn) nn = lr[2 * l + 1];

@@ -156,7 +156,7 @@ struct WalkBox {
   // kNoNode, and the sorted particle range of every cube
   const uint32_t *cube_node, *start_cube;
   float cpu, mass, inv_ll;
-  int n_cells, group_max;
+  int n_cells;
 };
 // Words of TreeBuffers::counters (64-bit ones take two).
 enum TreeCounter : int {
@@ -212,8 +212,10 @@ struct TreeParams {
   int group_level = 2;  // groups live in cubes of 2^level cells
 };
 
+// need: device word; the tree is built only where it is not zero (nullptr:
+// always). The level ranges start at zero.
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
-                TreeBuffers &tb, uint32_t *err, cudaStream_t st, int64_t *launches);
+                TreeBuffers &tb, const uint32_t *need, uint32_t *err, cudaStream_t st, int64_t *launches);
 void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb,
                  uint32_t *cube_start, int64_t ncubes, int cube_shift, cudaStream_t st,
                  int64_t *launches);
@@ -230,9 +232,9 @@ int64_t tree_scratch_words(int64_t np, int64_t ncubes);
 // where it applies, else every group of the tree walk.
 void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
                   cudaStream_t st, int64_t *launches);
-// The non-empty 4-cell cubes into tb.units (their count in tb.counters); the
-// direct summation's counterpart of tree_groups.
-void tree_units(TreeBuffers &tb, cudaStream_t st, int64_t *launches);
+// The 4-cell cubes to the direct summation (tb.units, kCntUnits) or the walk
+// (tb.groups, kCntGroups); the direct summation's counterpart of tree_groups.
+void tree_units(const TreeParams &tp, TreeBuffers &tb, cudaStream_t st, int64_t *launches);
 // The short-range law's columns on grids uniform in log r^2, indexed by the
 // float bits of s = r^2 + kLogR2Floor (cells^2). Entry k covers
 // [s_k, s_{k+1}), s_k the float whose top bits are (kLogBase + k) <<
@@ -270,8 +272,7 @@ struct LawTable {
   uint32_t cut_bits = 0xffffffffu;
 };
 // Direct summation over the units of every box (boxes: device array; uprefix:
-// their unit offsets when nbox > 1, unext: the queue head, zero): the cubes it
-// cannot take go to the boxes' group lists.
+// their unit offsets when nbox > 1, unext: the queue head, zero).
 void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, uint32_t *unext, uint32_t *stats,
                    const LawTable &law, float rsphere, cudaStream_t st);
 WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &tb, float *ftree,

@@ -309,7 +309,7 @@ int tpm_fof(tpm_ctx *c, float link, int32_t min_members, int32_t *labels, int me
   cudaStream_t st = c->st;
   int64_t np = c->np;
   // the sort and the octree of a force evaluation (no walk)
-  int rc = enqueue_forces(c, TPM_PART_TREE, st, false, false);
+  int rc = enqueue_forces(c, TPM_PART_TREE, st, false, false, true);
   if (rc) return rc;
   // five words per particle, reusing the caller-order force scratch and the
   // alternate sort buffers, which hold nothing between evaluations
@@ -319,7 +319,6 @@ int tpm_fof(tpm_ctx *c, float link, int32_t min_members, int32_t *labels, int me
   int32_t *out = reinterpret_cast<int32_t *>(c->fout);
   uint32_t *root = reinterpret_cast<uint32_t *>(c->fout) + np;
   uint32_t *ng = c->tb.counters + kCntFofGroups;
-  CK(cudaMemsetAsync(ng, 0, sizeof(uint32_t), st));
   k_fof_init<<<grid_of(np), 256, 0, st>>>(parent, gsize, label, np);
   int lb = (int)((np + kFofThreads - 1) / kFofThreads);
   if (lb > 148 * 32) lb = 148 * 32;

@@ -115,7 +115,9 @@ TPM_D uint32_t tb_levels(const TbShared<kItems> &sm, int t, int64_t i, int64_t n
 // Nodes per level and tile: cnt[l * ntiles + tile].
 template <int kItems>
 __global__ void __launch_bounds__(kTbThreads) k_tree_count(const uint64_t *__restrict__ key, int64_t np,
-                                                           uint32_t *__restrict__ cnt, int64_t ntiles) {
+                                                           uint32_t *__restrict__ cnt, int64_t ntiles,
+                                                           const uint32_t *__restrict__ need) {
+  if (need && *need == 0u) return;
   __shared__ TbShared<kItems> sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t base = blockIdx.x * (int64_t)sm.kTile;
@@ -145,7 +147,9 @@ __global__ void __launch_bounds__(kTbThreads) k_tree_count(const uint64_t *__res
 // One block per level: exclusive scan of the level's tile counts in place and
 // its total.
 __global__ void __launch_bounds__(1024) k_tree_scan(uint32_t *__restrict__ cnt, int64_t ntiles,
-                                                    uint32_t *__restrict__ total) {
+                                                    uint32_t *__restrict__ total,
+                                                    const uint32_t *__restrict__ need) {
+  if (need && *need == 0u) return;
   __shared__ uint32_t wsum[32];
   uint32_t *h = cnt + (int64_t)blockIdx.x * ntiles;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -244,7 +248,9 @@ template <int kItems>
 __global__ void __launch_bounds__(kTbThreads) k_tree_write(const uint64_t *__restrict__ key, int64_t np, TreeBuffers tb,
                                                            const uint32_t *__restrict__ cnt, int64_t ntiles,
                                                            const uint32_t *__restrict__ total, int cube_level,
-                                                           int sub_bits, double q_to_frac, uint32_t *err) {
+                                                           int sub_bits, double q_to_frac, uint32_t *err,
+                                                           const uint32_t *__restrict__ need) {
+  if (need && *need == 0u) return;
   __shared__ TbShared<kItems> sm;
   __shared__ TbNode queue[kTbWarps][kTbQueue];
   __shared__ uint32_t lbase[kTbLevels + 1];  // first node of each level
@@ -383,7 +389,9 @@ TPM_D void put_moments(const TreeBuffers &tb, uint32_t node, uint4 geo, const No
 // child index and its own; 0 for a node that does not split), and the moments
 // of those without, from their particles.
 __global__ void __launch_bounds__(256) k_tree_leaves(const uint32_t *__restrict__ spos, TreeBuffers tb, float cpu,
-                                                     float mass, float inv_theta2) {
+                                                     float mass, float inv_theta2,
+                                                     const uint32_t *__restrict__ need) {
+  if (need && *need == 0u) return;
   __shared__ uint32_t lr[2 * kTbLevels];
   if (threadIdx.x < 2 * kTbLevels) lr[threadIdx.x] = tb.level_range[threadIdx.x];
   __syncthreads();
@@ -490,28 +498,15 @@ TPM_D void inner_moments(const TreeBuffers &tb, uint32_t b, uint32_t e, uint32_t
   }
 }
 
-__global__ void __launch_bounds__(256) k_tree_inner(TreeBuffers tb, int l, float cpu, float inv_theta2) {
+__global__ void __launch_bounds__(256) k_tree_inner(TreeBuffers tb, int l, float cpu, float inv_theta2,
+                                                    const uint32_t *__restrict__ need) {
+  if (need && *need == 0u) return;
   inner_moments(tb, tb.level_range[2 * l], tb.level_range[2 * l + 1], (blockIdx.x * blockDim.x + threadIdx.x) >> 3,
                 (gridDim.x * blockDim.x) >> 3, cpu, inv_theta2);
 }
 
-// Levels lmax to 0 in one launch, one cluster of kTopBlocks blocks with its
-// hardware barrier between the levels.
-constexpr int kTopBlocks = 8;
-constexpr int kTopThreads = 512;
-__global__ void __cluster_dims__(kTopBlocks, 1, 1) __launch_bounds__(kTopThreads)
-    k_tree_top(TreeBuffers tb, int lmax, float cpu, float inv_theta2) {
-  for (int l = lmax; l >= 0; l--) {
-    inner_moments(tb, tb.level_range[2 * l], tb.level_range[2 * l + 1], (blockIdx.x * kTopThreads + threadIdx.x) >> 3,
-                  (kTopBlocks * kTopThreads) >> 3, cpu, inv_theta2);
-    __threadfence();
-    __syncthreads();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  }
-}
-
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
-                TreeBuffers &tb, uint32_t *err, cudaStream_t st, int64_t *launches) {
+                TreeBuffers &tb, const uint32_t *need, uint32_t *err, cudaStream_t st, int64_t *launches) {
   const int cbits = kAxisBits - tp.sub_bits;
   const int64_t ntiles = tree_tiles(np);
   uint32_t *cnt = tb.tile_sum, *total = cnt + kTbLevels * ntiles;
@@ -519,29 +514,26 @@ void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos,
   const double q_to_frac = 1.0 / ((double)(1u << tp.sub_bits) * (double)tp.n);
   const bool big = tb_items(np) == kTbItemsBig;
   if (big)
-    k_tree_count<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
+    k_tree_count<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles, need);
   else
-    k_tree_count<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
-  k_tree_scan<<<kTbLevels, 1024, 0, st>>>(cnt, ntiles, total);
+    k_tree_count<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles, need);
+  k_tree_scan<<<kTbLevels, 1024, 0, st>>>(cnt, ntiles, total, need);
   if (big)
     k_tree_write<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
-                                                                       tp.sub_bits, q_to_frac, err);
+                                                                       tp.sub_bits, q_to_frac, err, need);
   else
     k_tree_write<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
-                                                                         tp.sub_bits, q_to_frac, err);
+                                                                         tp.sub_bits, q_to_frac, err, need);
   float inv_theta2 = 1.f / tp.theta2;
   const int leaf_grid = (int)std::min<int64_t>((np + 255) / 256, kBuildGrid);
-  k_tree_leaves<<<leaf_grid, 256, 0, st>>>(spos, tb, tp.cell_per_unit, tp.mass, inv_theta2);
+  k_tree_leaves<<<leaf_grid, 256, 0, st>>>(spos, tb, tp.cell_per_unit, tp.mass, inv_theta2, need);
   int64_t nl = 4;
-  // the levels of at most 8 nodes per segment of the cluster in one launch,
-  // each deeper one in its own
-  int l = kAxisBits - 1;
-  for (; l > 4; l--) {
-    k_tree_inner<<<(int)std::min<int64_t>((np + 31) / 32, kBuildGrid), 256, 0, st>>>(tb, l, tp.cell_per_unit, inv_theta2);
+  // the walk starts at the 4-cell cubes and reads no moments above them
+  for (int l = kAxisBits - 1; l >= cbits - 2; l--) {
+    k_tree_inner<<<(int)std::min<int64_t>((np + 31) / 32, kBuildGrid), 256, 0, st>>>(tb, l, tp.cell_per_unit,
+                                                                                     inv_theta2, need);
     nl++;
   }
-  k_tree_top<<<kTopBlocks, kTopThreads, 0, st>>>(tb, l, tp.cell_per_unit, inv_theta2);
-  nl++;
   if (launches) *launches += nl;
 }
 
@@ -669,7 +661,7 @@ void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuff
 void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
                   cudaStream_t st, int64_t *launches) {
   if (direct_applies(tp)) {
-    tree_units(tb, st, launches);
+    tree_units(tp, tb, st, launches);
   } else {
     const int cbits = kAxisBits - tp.sub_bits;
     tree_groups(tp, key, np, tb, cube_start, 1ll << (3 * (cbits - tp.group_level)), 3 * (tp.sub_bits + tp.group_level),
@@ -1253,7 +1245,6 @@ WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &
   b.mass = tp.mass;
   b.inv_ll = (float)(1.0 / ((double)tp.n * (double)tp.n));
   b.n_cells = (int)tp.n;
-  b.group_max = std::max(1, std::min(32, tp.group_max));
   return b;
 }
 

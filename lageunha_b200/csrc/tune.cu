@@ -102,8 +102,8 @@ int tpm_autotune(tpm_ctx *c, unsigned what, tpm_tuning *out) {
   if (!c) return fail(TPM_E_ARG, "ctx is NULL");
   if (c->np <= 0) return fail(TPM_E_STATE, "no particles loaded");
   CK(cudaSetDevice(c->device));
-  // one evaluation leaves sorted keys, the mesh and the tree in place
-  int rc = enqueue_forces(c, TPM_PART_ALL, c->st, false);
+  // one evaluation leaves sorted keys, the mesh and the whole tree in place
+  int rc = enqueue_forces(c, TPM_PART_ALL, c->st, false, true, true);
   if (!rc) rc = finish_forces(c, TPM_PART_ALL, false, false);
   if (rc) return rc;
   tpm_tuning res;

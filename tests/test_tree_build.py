@@ -39,7 +39,7 @@ def test_groups_and_tree_force(kind, count):
         eng.load_fixed(pu)
         lab, ng = eng.fof(0.21, 2)
         t = eng.tuning
-        t.group_max = 16
+        t.group_level = 3  # every particle to the walk, which needs the tree
         eng.tuning = t
         eng.compute(E.PART_TREE)
         f = eng.forces().astype(np.float64)
