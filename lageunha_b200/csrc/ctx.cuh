@@ -46,6 +46,10 @@ struct tpm_ctx {
   // after the sort and joined before the walk, beside the tree build on st
   cudaStream_t st_pm = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // the direct short-range sum runs on st_dir, forked once its cubes are known,
+  // joined before the walk, beside the tree build and the PM chain
+  cudaStream_t st_dir = nullptr;
+  cudaEvent_t ev_dfork = nullptr, ev_djoin = nullptr;
   bool overlapped = false;  // the last timed evaluation ran the two chains side by side
   // streamed evaluations (tpm_stream_submit / tpm_stream_wait): two slots of
   // positions and forces, a copy-in and a copy-out stream

@@ -464,8 +464,8 @@ void tree_units(const TreeParams &tp, TreeBuffers &tb, cudaStream_t st, int64_t 
   if (launches) *launches += 1;
 }
 
-void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, uint32_t *unext, uint32_t *stats,
-                   const LawTable &law, float rsphere, cudaStream_t st) {
+void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, int64_t max_units, uint32_t *unext,
+                   uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st) {
   const size_t smem = sizeof(float4) * kLogSmemF4 + sizeof(DirTeam) * kDirTeams + sizeof(DirWarp) * kDirTeams * kDirWarps;
   static_assert(sizeof(DirTeam) % 16 == 0 && sizeof(DirWarp) % 16 == 0, "float4 alignment");
   static_assert(sizeof(float4) * kLogSmemF4 + sizeof(DirTeam) * kDirTeams + sizeof(DirWarp) * kDirTeams * kDirWarps <=
@@ -478,12 +478,15 @@ void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, uint
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // a block fills its SM, so blocks that would find no unit are left out: a
+  // small box's PM chain runs beside the sum on the SMs that remain
+  const int grid = (int)std::min<int64_t>(sms, (max_units + kDirTeams - 1) / kDirTeams);
   const float rs2 = rsphere * rsphere;
   const uint32_t kcut = law_cut_bin(law, rs2);
   if (law.hard_cut)
-    k_direct<true><<<sms, kDirThreads, smem, st>>>(boxes, uprefix, nbox, unext, stats, law.tlog, rsphere, kcut);
+    k_direct<true><<<grid, kDirThreads, smem, st>>>(boxes, uprefix, nbox, unext, stats, law.tlog, rsphere, kcut);
   else
-    k_direct<false><<<sms, kDirThreads, smem, st>>>(boxes, uprefix, nbox, unext, stats, law.tlog, rsphere, kcut);
+    k_direct<false><<<grid, kDirThreads, smem, st>>>(boxes, uprefix, nbox, unext, stats, law.tlog, rsphere, kcut);
 }
 
 }  // namespace tpm

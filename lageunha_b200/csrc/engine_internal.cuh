@@ -272,18 +272,21 @@ struct LawTable {
   uint32_t cut_bits = 0xffffffffu;
 };
 // Direct summation over the units of every box (boxes: device array; uprefix:
-// their unit offsets when nbox > 1, unext: the queue head, zero).
-void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, uint32_t *unext, uint32_t *stats,
-                   const LawTable &law, float rsphere, cudaStream_t st);
+// their unit offsets when nbox > 1, max_units: a bound on the units of all,
+// unext: the queue head, zero).
+void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, int64_t max_units, uint32_t *unext,
+                   uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st);
 WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &tb, float *ftree,
                  uint32_t *err);
 // One launch over the groups of every box (boxes: device array); the boxes
 // share law (same kind, softening, split and cut) and rsphere.
 void tree_walk_multi(const WalkBox *boxes, int nbox, uint32_t *gprefix, uint32_t *gnext, uint32_t *stack,
                      int64_t stack_words, uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st);
-void tree_walk(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb,
-               const LawTable &law, float *ftree, uint32_t *err, cudaStream_t st,
-               int64_t *launches);
+// The box record and the direct summation over tb.units; needs no tree.
+void tree_direct(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb, const LawTable &law,
+                 float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches);
+// The walk over tb.groups, after tree_build and the record that tree_direct set.
+void tree_walk(const TreeParams &tp, const TreeBuffers &tb, const LawTable &law, cudaStream_t st, int64_t *launches);
 
 // ---------------------------------------------------------------- misc
 // Sets the message tpm_last_error() returns on this thread.

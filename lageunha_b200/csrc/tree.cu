@@ -1268,18 +1268,23 @@ __global__ void k_set_walkbox(WalkBox *dst, WalkBox v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *dst = v;
 }
 
-void tree_walk(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb,
-               const LawTable &law, float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches) {
-  (void)np;
-  // the box record goes to the device with the launch that precedes the walk
+void tree_direct(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb, const LawTable &law,
+                 float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches) {
+  // the box record goes to the device with the launch that precedes the sum
   k_set_walkbox<<<1, 32, 0, st>>>(tb.walkbox, walk_box(tp, spos, tb, ftree, err));
+  if (launches) *launches += 1;
   // the next-item counters were zeroed before tree_groups / tree_units
   if (direct_applies(tp)) {
-    launch_direct(tb.walkbox, nullptr, 1, &tb.counters[kCntNextUnit], tb.counters, law, tp.rsphere, st);
+    launch_direct(tb.walkbox, nullptr, 1, std::min(np, tb.ncubes4), &tb.counters[kCntNextUnit], tb.counters, law,
+                  tp.rsphere, st);
     if (launches) *launches += 1;
   }
-  launch_walk(tb.walkbox, nullptr, 1, &tb.counters[kCntNextGroup], tb.stack, tb.stack_words, tb.counters, law, tp.rsphere, st);
-  if (launches) *launches += 2;
+}
+
+void tree_walk(const TreeParams &tp, const TreeBuffers &tb, const LawTable &law, cudaStream_t st, int64_t *launches) {
+  launch_walk(tb.walkbox, nullptr, 1, &tb.counters[kCntNextGroup], tb.stack, tb.stack_words, tb.counters, law,
+              tp.rsphere, st);
+  if (launches) *launches += 1;
 }
 
 // Prefix of the boxes' group (or unit) counts, counters[word], and the
@@ -1302,7 +1307,7 @@ void tree_walk_multi(const WalkBox *boxes, int nbox, uint32_t *gprefix, uint32_t
   // every box's direct summation first: it leaves the groups of the cubes it
   // cannot take in the boxes' group lists
   k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntUnits, gprefix, gnext);
-  launch_direct(boxes, gprefix, nbox, gnext, stats, law, rsphere, st);
+  launch_direct(boxes, gprefix, nbox, 1ll << 40, gnext, stats, law, rsphere, st);
   k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntGroups, gprefix, gnext);
   launch_walk(boxes, gprefix, nbox, gnext, stack, stack_words, stats, law, rsphere, st);
 }

@@ -68,7 +68,8 @@ void groups_and_walk(tpm_ctx *c) {
   TreeParams tp = tree_params(c);
   cudaMemsetAsync(c->tb.counters, 0, sizeof(uint32_t) * 16, c->st);
   tree_targets(tp, c->skey, c->np, c->tb, c->cube_start, c->st, nullptr);
-  tree_walk(tp, c->spos, c->np, c->tb, c->law, c->ftree, c->err, c->st, nullptr);
+  tree_direct(tp, c->spos, c->np, c->tb, c->law, c->ftree, c->err, c->st, nullptr);
+  tree_walk(tp, c->tb, c->law, c->st, nullptr);
 }
 
 }  // namespace
