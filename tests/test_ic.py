@@ -118,6 +118,57 @@ def test_engine_noise_matches_reference(n, seed, weighted):
     assert _noise_close(got, want) < 1e-4
 
 
+def ran3_values(idum, count):
+    """The first `count` states of ran3, x_t = x_(t-55) - x_(t-24) mod 10^9, 24 at a time."""
+    st = O._ran3_stream(idum)
+    x = np.empty(count, np.int64)
+    m = min(55, count)
+    x[:m] = [next(st) for _ in range(m)]
+    for t in range(m, count, 24):
+        e = min(24, count - t)
+        x[t:t + e] = x[t - 55:t - 55 + e] - x[t - 24:t - 24 + e]
+        x[t:t + e] += (x[t:t + e] < 0) * 10 ** 9
+    return x
+
+
+def gasdev_values(idum, count):
+    """O.gasdev_pairs on whole arrays, for large counts."""
+    f32 = np.float32
+    # a trial is accepted with probability pi / 4; 8 standard deviations of slack
+    trials = int(count * 4 / np.pi + 8 * np.sqrt(count) + 64)
+    u = (ran3_values(idum, 2 * trials) * (1.0 / 1e9)).astype(f32)
+    v = (2.0 * u.astype(np.float64) - 1.0).astype(f32).reshape(-1, 2)
+    rsq = v[:, 0] * v[:, 0] + v[:, 1] * v[:, 1]
+    ok = np.nonzero((rsq < 1.0) & (rsq != 0.0))[0][:count]
+    assert len(ok) == count
+    r = rsq[ok].astype(np.float64)
+    fac = np.sqrt(-2.0 * np.log(r) / r).astype(f32)
+    return v[ok][:, ::-1] * fac[:, None]
+
+
+def test_array_restatement_matches_the_scalar_one():
+    assert np.array_equal(gasdev_values(-7, 700), O.gasdev_pairs(-7, 700))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,seed", [(12, -3), (24, -5), (72, -11), (256, -2024)])
+def test_engine_noise_across_jump_levels(n, seed):
+    """One jump start serves 110 trials, 32 starts hang from one of the level
+    above: 5, 42, 1131 and 50,000 starts cross each of the three levels. The
+    modes with kx > 0, which take the deviates as drawn; tolerance as above."""
+    k = np.fft.fftfreq(n, 1 / n).astype(np.int64)
+    k[n // 2] = n // 2
+    kx = np.arange(n // 2 + 1)
+    x = k[:, None, None] ** 2 + k[None, :, None] ** 2 + kx[None, None, :] ** 2
+    mask = (x > 0) & (x <= (n // 2) ** 2)
+    g = gasdev_values(seed, int(mask.sum()))
+    want = np.zeros(mask.shape, np.complex64)
+    want[mask] = g[:, 0] + 1j * g[:, 1]
+    got = E.ic_noise(n, seed, np.ones((n // 2) ** 2 + 1, np.float32))
+    assert got.shape == want.shape
+    assert _noise_close(got[:, :, 1:], want[:, :, 1:]) < 1e-4
+
+
 def _ref_particles(n, seed, vp, fnl, gnl, vamp, pfact):
     fx, fy, fz = O.ref_zeldovich(n, O.ref_ic_noise(n, seed, vp), fnl, gnl)
     f32 = np.float32
