@@ -205,6 +205,9 @@ def run_ic(E, ic, n, local):
 
 
 def cpu_baseline(workload):
+    from oracle import oracle as O
+    if not O.ref_available(O.VARIANT_A):
+        return {"unavailable": "oracle/_ref/libref_A.so was not built"}
     ps = reference_sample(workload)
     saved = _quiet_stdout()
     try:
