@@ -763,9 +763,11 @@ def run_engine_arm(args):
     if dominant == "tree_walk":
         flops = FLOP_PP * counters["pp"] + FLOP_PC * counters["pc"]
         achieved = flops / (per["tree_walk"] * 1e-3) / 1e12
-        tr = traffic.get("k_tree_walk")
-        roofline = {"bound": "fp32", "kernel": "k_tree_walk", "achieved": achieved, "peak": fp32_peak,
-                    "unit": "TFLOP/s", "frac": achieved / fp32_peak,
+        # the stage holds the direct sum and the walk of what it leaves
+        tr = traffic.get("k_direct")
+        roofline = {"bound": "fp32", "kernel": "k_direct" if counters["pc"] == 0 else "k_direct, k_tree_walk",
+                    "achieved": achieved,
+                    "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                     "peak_source": f"nominal FP32 {nsm} SMs x 128 lanes x 2 x {sm_max:.0f} MHz "
                                    "(no measured FP32 figure; HBM peak of measured)",
                     "traffic": (tr[0] * npart / tr[1]) if tr else None,
@@ -779,7 +781,10 @@ def run_engine_arm(args):
     # deposit, read and written once per transform, read by fda4
     grids = 1 if args.law == "reference" else 2
     mesh_pp = 4 * n ** 3 / npart
-    bytes_pp = {"sort": 28 + 5 * 32, "deposit": 12 + grids * mesh_pp, "fft": grids * 4 * mesh_pp,
+    # the sort: positions read for the counts and for the first pass, which writes
+    # 32-bit keys and indices; four passes read and write them; the gather reads
+    # index and position and writes position and key
+    bytes_pp = {"sort": 12 + 20 + 4 * 16 + 36, "deposit": 12 + grids * mesh_pp, "fft": grids * 4 * mesh_pp,
                 "fda4": 24 + grids * mesh_pp}
     hbm_stages = {}
     for k, b in bytes_pp.items():

@@ -1284,10 +1284,10 @@ TPM_D void fda_node_gradients(const float *boxf, float *gx, float *gy, float *gz
 // The force at one particle: its 27 nodes' gradients with the TSC weights
 // (fda4.h:46-54, 67-102, 276-292), relative to the tile's first node t - 1. The
 // nodes of each axis are taken in the order near, near + 1, near - 1 for every
-// particle, so that a load's lanes keep the offsets of their near nodes: with
-// the reference's near + sign, near - sign, which differ from lane to lane, a
-// load met 2.6 lanes to a bank, so 2.0. Bound by the shared-memory pipe, 80%
-// busy: 6.71 -> 6.37 ms for both grids of 512^3.
+// particle, so that a load's lanes keep the offsets of their near nodes; the
+// reference's near + sign, near - sign differ from lane to lane. Bound by the
+// shared-memory pipe (80% busy; 216M -> 194M wavefronts for both grids of 256^3
+// in this order): 6.71 -> 6.37 ms for both grids of 512^3.
 TPM_D float3 fda_interp(const float *gx, const float *gy, const float *gz, uint32_t ux, uint32_t uy, uint32_t uz,
                         uint32_t n, uint32_t half, int x0, int y0, int z0) {
   Axis ax = axis_of(ux, n, half), ay = axis_of(uy, n, half), az = axis_of(uz, n, half);
