@@ -763,11 +763,9 @@ def run_engine_arm(args):
     if dominant == "tree_walk":
         flops = FLOP_PP * counters["pp"] + FLOP_PC * counters["pc"]
         achieved = flops / (per["tree_walk"] * 1e-3) / 1e12
-        # the stage holds the direct sum and the walk of what it leaves
-        tr = traffic.get("k_direct")
-        roofline = {"bound": "fp32", "kernel": "k_direct" if counters["pc"] == 0 else "k_direct, k_tree_walk",
-                    "achieved": achieved,
-                    "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
+        tr = traffic.get("k_tree_walk")
+        roofline = {"bound": "fp32", "kernel": "k_tree_walk", "achieved": achieved, "peak": fp32_peak,
+                    "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                     "peak_source": f"nominal FP32 {nsm} SMs x 128 lanes x 2 x {sm_max:.0f} MHz "
                                    "(no measured FP32 figure; HBM peak of measured)",
                     "traffic": (tr[0] * npart / tr[1]) if tr else None,

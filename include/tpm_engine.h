@@ -390,13 +390,10 @@ int tpm_ewald(tpm_ctx *ctx, int64_t nt, const int64_t *targets, double *out);
 /* Per-stage device times (ms) of the last tpm_compute_forces, in the order
  * sort, deposit, fft, fda4, tree_build, tree_walk, finish; returns the
  * number of stages written (<= n). Where the chains run side by side the
- * times overlap: tree_build lasts until the mesh chain is done too, and in
- * boxes below 4M particles the direct short-range sum runs beside both, so
- * tree_walk holds only what remains of it. */
+ * times overlap: tree_build lasts until the mesh chain is done too. */
 int tpm_stage_times(tpm_ctx *ctx, float *ms, int n);
 
-/* Counters of the last force evaluation: [0] tree nodes (0 where the direct
- * summation took every cube and no tree was needed), [1] particle-
+/* Counters of the last force evaluation: [0] tree nodes, [1] particle-
  * particle interactions, [2] particle-node interactions, [3] walk groups,
  * [4] walk iterations, [5] nodes examined by the walk, [6] deepest walk stack. */
 int tpm_counters(tpm_ctx *ctx, int64_t *out, int n);

@@ -46,10 +46,6 @@ struct tpm_ctx {
   // after the sort and joined before the walk, beside the tree build on st
   cudaStream_t st_pm = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // the direct short-range sum runs on st_dir, forked once its cubes are known,
-  // joined before the walk, beside the tree build and the PM chain
-  cudaStream_t st_dir = nullptr;
-  cudaEvent_t ev_dfork = nullptr, ev_djoin = nullptr;
   bool overlapped = false;  // the last timed evaluation ran the two chains side by side
   // streamed evaluations (tpm_stream_submit / tpm_stream_wait): two slots of
   // positions and forces, a copy-in and a copy-out stream
@@ -142,9 +138,8 @@ const std::string &last_error_string();
 // Enqueues one force evaluation of the loaded particles on st (no host
 // synchronisation); with timing, records the stage events. walk == false
 // stops before the tree walk (the tree and the groups are built): an
-// ensemble walks all its boxes in one launch. The tree is built where the
-// direct summation leaves groups to the walk, or always with whole_tree.
-int enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk = true, bool whole_tree = false);
+// ensemble walks all its boxes in one launch.
+int enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk = true);
 // The walk record of the context's current buffers.
 WalkBox ctx_walk_box(const tpm_ctx *c);
 // After the stream has finished an evaluation: checks the device error words

@@ -128,7 +128,6 @@ static void quiesce(tpm_ctx *c) {
   if (!c->arena) return;
   if (c->st) cudaStreamSynchronize(c->st);
   if (c->st_pm) cudaStreamSynchronize(c->st_pm);
-  if (c->st_dir) cudaStreamSynchronize(c->st_dir);
   if (c->sp.in) cudaStreamSynchronize(c->sp.in);
   if (c->sp.out) cudaStreamSynchronize(c->sp.out);
 }
@@ -302,7 +301,6 @@ static int alloc_mesh(tpm_ctx *c) {
   CK(cudaMemsetAsync(c->phi, 0, sizeof(float) * (int64_t)g.px * g.py * g.pz, c->st));
   c->ncubes = 1ll << (3 * (g.cbits - 2));
   CK(dmalloc(c->arena, &c->cube_start, sizeof(uint32_t) * (c->ncubes + 1)));
-  c->tb.units = c->cube_start;
   c->tb.ncubes4 = c->ncubes;
   CK(dmalloc(c->arena, &c->tb.cube_node, sizeof(uint32_t) * c->ncubes));
   CK(dmalloc(c->arena, &c->tb.start_cube, sizeof(uint32_t) * (c->ncubes + 1)));
@@ -593,10 +591,7 @@ int tpm::create_ctx(const tpm_params *params, int device, DeviceArena *arena, tp
   {
     if (cudaStreamCreateWithFlags(&c->st_pm, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->st_dir, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_dfork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_djoin, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
       tpm_destroy(c);
       return fail(TPM_E_CUDA, "stream or event creation failed");
     }
@@ -662,10 +657,7 @@ int tpm_destroy(tpm_ctx *c) {
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
-  if (c->ev_dfork) cudaEventDestroy(c->ev_dfork);
-  if (c->ev_djoin) cudaEventDestroy(c->ev_djoin);
   if (c->st_pm) cudaStreamDestroy(c->st_pm);
-  if (c->st_dir) cudaStreamDestroy(c->st_dir);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
   return 0;
@@ -755,14 +747,7 @@ int tpm_load_lagrangian(tpm_ctx *c, int64_t np, const void *particles, int64_t s
 
 }  // extern "C"
 
-// Below this many particles the direct sum runs beside the PM chain and the
-// tree build: it leaves SMs idle (512 cubes at 32^3 take 103 of 148) or has a
-// long tail. 32^3 captured 225 -> 178 us, 64^3 495 -> 458 us, 128^3 step 2.63 ->
-// 2.57 ms. Above, it fills the device and both take turns (512^3: 0.5%), so it
-// follows them and the stage times stay apart.
-constexpr int64_t kDirectBeside = 1 << 22;
-
-int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk, bool whole_tree) {
+int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing, bool walk) {
   const MeshGeom &g = c->g;
   int64_t np = c->np;
   c->launches = 0;
@@ -842,32 +827,17 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
     tp.mass = c->prm.particle_mass;
     tp.group_max = c->tune_group_max;
     tp.group_level = c->tune_group_level;
-    tree_targets(tp, c->skey, np, c->tb, c->cube_start, st, &c->launches);
-    const bool beside = walk && np < kDirectBeside;
-    if (beside) {
-      // the direct sum needs no tree: it starts beside the PM chain and the
-      // build (whose kernels return at once where no group is left to the walk)
-      CK(cudaEventRecord(c->ev_dfork, st));
-      CK(cudaStreamWaitEvent(c->st_dir, c->ev_dfork, 0));
-      tree_direct(tp, c->spos, np, c->tb, c->law, c->ftree, c->err, c->st_dir, &c->launches);
-      CK(cudaEventRecord(c->ev_djoin, c->st_dir));
-    }
-    tree_build(tp, c->skey, c->spos, np, c->tb, whole_tree ? nullptr : &c->tb.counters[kCntGroups], c->err, st,
-               &c->launches);
+    tree_build(tp, c->skey, c->spos, np, c->tb, c->err, st, &c->launches);
+    tree_groups(tp, c->skey, np, c->tb, c->cube_start, st, &c->launches);
     CK(stage_check(st, "tree_build"));
-    // the tree_build stage of an overlapped evaluation ends with the PM chain
+    // the walk takes every SM: it starts once the PM chain is done too (the
+    // tree_build stage of an overlapped evaluation ends with both chains)
     if (split) {
       CK(cudaStreamWaitEvent(st, c->ev_join, 0));
       split = false;
     }
     if (timing) CK(cudaEventRecord(c->ev[5], st));
-    if (walk) {
-      if (beside)
-        CK(cudaStreamWaitEvent(st, c->ev_djoin, 0));
-      else
-        tree_direct(tp, c->spos, np, c->tb, c->law, c->ftree, c->err, st, &c->launches);
-      tree_walk(tp, c->tb, c->law, st, &c->launches);
-    }
+    if (walk) tree_walk(tp, c->spos, np, c->tb, c->law, c->ftree, c->err, st, &c->launches);
     CK(stage_check(st, "tree_walk"));
     if (timing) CK(cudaEventRecord(c->ev[6], st));
   } else if (timing) {
@@ -910,7 +880,7 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
     auto wide = [&](int w) { return (int64_t)(((uint64_t)hc[w + 1] << 32) | hc[w]); };
     c->counters[1] = wide(kCntPp);
     c->counters[2] = wide(kCntPc);
-    c->counters[3] = (int64_t)hc[kCntGroups] + hc[kCntSubs];
+    c->counters[3] = hc[kCntGroups];
     c->counters[4] = wide(kCntIter);
     c->counters[5] = wide(kCntVisit);
     c->counters[6] = hc[kCntMaxTop];

@@ -146,9 +146,8 @@ struct WalkBox {
   const uint32_t *spos;
   const uint4 *walkA, *walkB;
   const float4 *mom0, *mom1, *mom2;
-  uint32_t *groups;         // the groups the walk takes: start, count pairs
-  const uint32_t *units;    // the non-empty 4-cell cubes of the direct summation
-  uint32_t *counters;       // device words, TreeCounter
+  const uint32_t *groups;    // start, count pairs
+  const uint32_t *counters;  // device words, TreeCounter
   float *ftree;
   uint32_t *err;
   // where each group's walk starts: the 4-cell cubes of the tree's level
@@ -167,10 +166,7 @@ enum TreeCounter : int {
   kCntIter = 6,       // walk iterations (64 bits)
   kCntVisit = 8,      // nodes the walk examined (64 bits)
   kCntMaxTop = 10,    // deepest walk stack
-  kCntUnits = 11,     // cubes of the direct summation
-  kCntFofGroups = 12,
-  kCntNextUnit = 13,  // the direct summation's queue head
-  kCntSubs = 14       // its target sub-groups
+  kCntFofGroups = 12
 };
 constexpr uint32_t kNoNode = 0xffffffffu;
 struct TreeBuffers {
@@ -189,7 +185,6 @@ struct TreeBuffers {
   uint32_t *groups = nullptr;       // walk groups: start | (count << 26) packed as 2 words
   int64_t cap_groups = 0;
   uint32_t *counters = nullptr;     // [16], TreeCounter
-  uint32_t *units = nullptr;        // the context's cube_start buffer (ncubes4 words)
   uint32_t *stack = nullptr;        // per-warp global stacks
   int64_t stack_words = 0;
   WalkBox *walkbox = nullptr;       // device copy of this box's walk record
@@ -212,29 +207,15 @@ struct TreeParams {
   int group_level = 2;  // groups live in cubes of 2^level cells
 };
 
-// need: device word; the tree is built only where it is not zero (nullptr:
-// always). The level ranges start at zero.
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
-                TreeBuffers &tb, const uint32_t *need, uint32_t *err, cudaStream_t st, int64_t *launches);
-void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb,
-                 uint32_t *cube_start, int64_t ncubes, int cube_shift, cudaStream_t st,
-                 int64_t *launches);
-// Whether a box's short-range force starts with the direct summation over
-// its 4-cell cubes (direct.cu): the groups are cut from those cubes, and a
-// cube's reach stays within half a box of any of its targets.
-inline bool direct_applies(const TreeParams &tp) {
-  return tp.group_level == 2 && (float)tp.n >= 2.f * (4.f + tp.rsphere);
-}
+                TreeBuffers &tb, uint32_t *err, cudaStream_t st, int64_t *launches);
+// The groups of the walk, cut from the cubes of group_level (cube_start:
+// scratch for their range table where they are not the 4-cell ones).
+void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
+                 cudaStream_t st, int64_t *launches);
 // Words of TreeBuffers::tile_sum: the build's counts per level and tile, or the
 // group counts and offsets of a mesh with ncubes 4-cell cubes.
 int64_t tree_scratch_words(int64_t np, int64_t ncubes);
-// What the short-range force iterates over: the units of the direct summation
-// where it applies, else every group of the tree walk.
-void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
-                  cudaStream_t st, int64_t *launches);
-// The 4-cell cubes to the direct summation (tb.units, kCntUnits) or the walk
-// (tb.groups, kCntGroups); the direct summation's counterpart of tree_groups.
-void tree_units(const TreeParams &tp, TreeBuffers &tb, cudaStream_t st, int64_t *launches);
 // The short-range law's columns on grids uniform in log r^2, indexed by the
 // float bits of s = r^2 + kLogR2Floor (cells^2). Entry k covers
 // [s_k, s_{k+1}), s_k the float whose top bits are (kLogBase + k) <<
@@ -271,22 +252,15 @@ struct LawTable {
   // zero entry)
   uint32_t cut_bits = 0xffffffffu;
 };
-// Direct summation over the units of every box (boxes: device array; uprefix:
-// their unit offsets when nbox > 1, max_units: a bound on the units of all,
-// unext: the queue head, zero).
-void launch_direct(const WalkBox *boxes, const uint32_t *uprefix, int nbox, int64_t max_units, uint32_t *unext,
-                   uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st);
 WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &tb, float *ftree,
                  uint32_t *err);
 // One launch over the groups of every box (boxes: device array); the boxes
 // share law (same kind, softening, split and cut) and rsphere.
 void tree_walk_multi(const WalkBox *boxes, int nbox, uint32_t *gprefix, uint32_t *gnext, uint32_t *stack,
                      int64_t stack_words, uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st);
-// The box record and the direct summation over tb.units; needs no tree.
-void tree_direct(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb, const LawTable &law,
-                 float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches);
-// The walk over tb.groups, after tree_build and the record that tree_direct set.
-void tree_walk(const TreeParams &tp, const TreeBuffers &tb, const LawTable &law, cudaStream_t st, int64_t *launches);
+void tree_walk(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb,
+               const LawTable &law, float *ftree, uint32_t *err, cudaStream_t st,
+               int64_t *launches);
 
 // ---------------------------------------------------------------- misc
 // Sets the message tpm_last_error() returns on this thread.

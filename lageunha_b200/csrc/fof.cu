@@ -309,7 +309,7 @@ int tpm_fof(tpm_ctx *c, float link, int32_t min_members, int32_t *labels, int me
   cudaStream_t st = c->st;
   int64_t np = c->np;
   // the sort and the octree of a force evaluation (no walk)
-  int rc = enqueue_forces(c, TPM_PART_TREE, st, false, false, true);
+  int rc = enqueue_forces(c, TPM_PART_TREE, st, false, false);
   if (rc) return rc;
   // five words per particle, reusing the caller-order force scratch and the
   // alternate sort buffers, which hold nothing between evaluations

@@ -1,5 +1,5 @@
-// The short-range pair law and the cube geometry shared by the direct
-// summation (direct.cu) and the tree walk (tree.cu).
+// The short-range pair law of the tree walk (tree.cu) and the cube geometry it
+// shares with the search for groups (fof.cu).
 #pragma once
 #include <string.h>
 
@@ -115,30 +115,6 @@ TPM_D void axis_runs(float lo, float hi, int n, int run[4]) {
   run[1] = ncube - a;
   run[2] = 0;
   run[3] = b + 1;
-}
-
-// Every third bit of c, from bit 0 (c < 2^30).
-TPM_D uint32_t compact3(uint32_t c) {
-  c &= 0x09249249u;
-  c = (c ^ (c >> 2)) & 0x030c30c3u;
-  c = (c ^ (c >> 4)) & 0x0300f00fu;
-  c = (c ^ (c >> 8)) & 0x030000ffu;
-  c = (c ^ (c >> 16)) & 0x000003ffu;
-  return c;
-}
-
-// Cubes that only touch the reach (rsphere a multiple of four) hold no particle
-// inside it: cube faces are whole cells, exact in float, so the runs of cubes in
-// reach end just short of it.
-constexpr float kCubeReach = 0.999999f;
-
-// The gap along one axis of an n-cell periodic box between 4-cell cube c and a
-// box of half width hw about mid (cells), minimum image.
-TPM_D float cube_gap(int c, float mid, float hw, int n, float inv_n) {
-  const float lo = (float)(4 * c), hi = (float)min(4 * c + 4, n);
-  float d = 0.5f * (lo + hi) - mid;
-  d -= (float)n * rintf(d * inv_n);
-  return fmaxf(fabsf(d) - 0.5f * (hi - lo) - hw, 0.f);
 }
 
 }  // namespace tpm

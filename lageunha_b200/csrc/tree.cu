@@ -115,9 +115,7 @@ TPM_D uint32_t tb_levels(const TbShared<kItems> &sm, int t, int64_t i, int64_t n
 // Nodes per level and tile: cnt[l * ntiles + tile].
 template <int kItems>
 __global__ void __launch_bounds__(kTbThreads) k_tree_count(const uint64_t *__restrict__ key, int64_t np,
-                                                           uint32_t *__restrict__ cnt, int64_t ntiles,
-                                                           const uint32_t *__restrict__ need) {
-  if (need && *need == 0u) return;
+                                                           uint32_t *__restrict__ cnt, int64_t ntiles) {
   __shared__ TbShared<kItems> sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t base = blockIdx.x * (int64_t)sm.kTile;
@@ -147,9 +145,7 @@ __global__ void __launch_bounds__(kTbThreads) k_tree_count(const uint64_t *__res
 // One block per level: exclusive scan of the level's tile counts in place and
 // its total.
 __global__ void __launch_bounds__(1024) k_tree_scan(uint32_t *__restrict__ cnt, int64_t ntiles,
-                                                    uint32_t *__restrict__ total,
-                                                    const uint32_t *__restrict__ need) {
-  if (need && *need == 0u) return;
+                                                    uint32_t *__restrict__ total) {
   __shared__ uint32_t wsum[32];
   uint32_t *h = cnt + (int64_t)blockIdx.x * ntiles;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -248,9 +244,7 @@ template <int kItems>
 __global__ void __launch_bounds__(kTbThreads) k_tree_write(const uint64_t *__restrict__ key, int64_t np, TreeBuffers tb,
                                                            const uint32_t *__restrict__ cnt, int64_t ntiles,
                                                            const uint32_t *__restrict__ total, int cube_level,
-                                                           int sub_bits, double q_to_frac, uint32_t *err,
-                                                           const uint32_t *__restrict__ need) {
-  if (need && *need == 0u) return;
+                                                           int sub_bits, double q_to_frac, uint32_t *err) {
   __shared__ TbShared<kItems> sm;
   __shared__ TbNode queue[kTbWarps][kTbQueue];
   __shared__ uint32_t lbase[kTbLevels + 1];  // first node of each level
@@ -389,9 +383,7 @@ TPM_D void put_moments(const TreeBuffers &tb, uint32_t node, uint4 geo, const No
 // child index and its own; 0 for a node that does not split), and the moments
 // of those without, from their particles.
 __global__ void __launch_bounds__(256) k_tree_leaves(const uint32_t *__restrict__ spos, TreeBuffers tb, float cpu,
-                                                     float mass, float inv_theta2,
-                                                     const uint32_t *__restrict__ need) {
-  if (need && *need == 0u) return;
+                                                     float mass, float inv_theta2) {
   __shared__ uint32_t lr[2 * kTbLevels];
   if (threadIdx.x < 2 * kTbLevels) lr[threadIdx.x] = tb.level_range[threadIdx.x];
   __syncthreads();
@@ -498,15 +490,13 @@ TPM_D void inner_moments(const TreeBuffers &tb, uint32_t b, uint32_t e, uint32_t
   }
 }
 
-__global__ void __launch_bounds__(256) k_tree_inner(TreeBuffers tb, int l, float cpu, float inv_theta2,
-                                                    const uint32_t *__restrict__ need) {
-  if (need && *need == 0u) return;
+__global__ void __launch_bounds__(256) k_tree_inner(TreeBuffers tb, int l, float cpu, float inv_theta2) {
   inner_moments(tb, tb.level_range[2 * l], tb.level_range[2 * l + 1], (blockIdx.x * blockDim.x + threadIdx.x) >> 3,
                 (gridDim.x * blockDim.x) >> 3, cpu, inv_theta2);
 }
 
 void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos, int64_t np,
-                TreeBuffers &tb, const uint32_t *need, uint32_t *err, cudaStream_t st, int64_t *launches) {
+                TreeBuffers &tb, uint32_t *err, cudaStream_t st, int64_t *launches) {
   const int cbits = kAxisBits - tp.sub_bits;
   const int64_t ntiles = tree_tiles(np);
   uint32_t *cnt = tb.tile_sum, *total = cnt + kTbLevels * ntiles;
@@ -514,24 +504,24 @@ void tree_build(const TreeParams &tp, const uint64_t *key, const uint32_t *spos,
   const double q_to_frac = 1.0 / ((double)(1u << tp.sub_bits) * (double)tp.n);
   const bool big = tb_items(np) == kTbItemsBig;
   if (big)
-    k_tree_count<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles, need);
+    k_tree_count<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
   else
-    k_tree_count<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles, need);
-  k_tree_scan<<<kTbLevels, 1024, 0, st>>>(cnt, ntiles, total, need);
+    k_tree_count<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, cnt, ntiles);
+  k_tree_scan<<<kTbLevels, 1024, 0, st>>>(cnt, ntiles, total);
   if (big)
     k_tree_write<kTbItemsBig><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
-                                                                       tp.sub_bits, q_to_frac, err, need);
+                                                                       tp.sub_bits, q_to_frac, err);
   else
     k_tree_write<kTbItemsSmall><<<(unsigned)ntiles, kTbThreads, 0, st>>>(key, np, tb, cnt, ntiles, total, cbits - 2,
-                                                                         tp.sub_bits, q_to_frac, err, need);
+                                                                         tp.sub_bits, q_to_frac, err);
   float inv_theta2 = 1.f / tp.theta2;
   const int leaf_grid = (int)std::min<int64_t>((np + 255) / 256, kBuildGrid);
-  k_tree_leaves<<<leaf_grid, 256, 0, st>>>(spos, tb, tp.cell_per_unit, tp.mass, inv_theta2, need);
+  k_tree_leaves<<<leaf_grid, 256, 0, st>>>(spos, tb, tp.cell_per_unit, tp.mass, inv_theta2);
   int64_t nl = 4;
   // the walk starts at the 4-cell cubes and reads no moments above them
   for (int l = kAxisBits - 1; l >= cbits - 2; l--) {
     k_tree_inner<<<(int)std::min<int64_t>((np + 31) / 32, kBuildGrid), 256, 0, st>>>(tb, l, tp.cell_per_unit,
-                                                                                     inv_theta2, need);
+                                                                                     inv_theta2);
     nl++;
   }
   if (launches) *launches += nl;
@@ -639,11 +629,16 @@ void scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *bsum, uint
   k_scan_sums<<<1, 1024, 0, st>>>(bsum, nb, total);
 }
 
-void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb,
-                 uint32_t *cube_start, int64_t ncubes, int cube_shift, cudaStream_t st,
-                 int64_t *launches) {
+void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
+                 cudaStream_t st, int64_t *launches) {
   uint32_t gmax = (uint32_t)std::max(1, std::min(32, tp.group_max));
-  launch_range_table(key, np, cube_shift, (uint32_t)ncubes, cube_start, st);
+  const int64_t ncubes = 1ll << (3 * (kAxisBits - tp.sub_bits - tp.group_level));
+  const uint32_t *start = tb.start_cube;  // of the 4-cell cubes
+  if (tp.group_level != 2) {
+    launch_range_table(key, np, 3 * (tp.sub_bits + tp.group_level), (uint32_t)ncubes, cube_start, st);
+    if (launches) *launches += 1;
+    start = cube_start;
+  }
   // gcount and offsets live in the tail of the group buffer's scratch
   uint32_t *gcount = tb.tile_sum;  // sized >= ncubes + blocks by the caller
   uint32_t *goff = gcount + ncubes;
@@ -651,22 +646,11 @@ void tree_groups(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuff
   uint32_t *bsum = goff + ncubes;
   int blocks = (int)((ncubes + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_group_counts<<<blocks, 256, 0, st>>>(cube_start, ncubes, gcount, gmax);
+  k_group_counts<<<blocks, 256, 0, st>>>(start, ncubes, gcount, gmax);
   k_scan_block<<<(unsigned)nb, 1024, 0, st>>>(gcount, goff, ncubes, bsum);
   k_scan_sums<<<1, 1024, 0, st>>>(bsum, nb, &tb.counters[kCntGroups]);
-  k_write_groups<<<blocks, 256, 0, st>>>(cube_start, ncubes, goff, bsum, tb.groups, gmax);
-  if (launches) *launches += 5;
-}
-
-void tree_targets(const TreeParams &tp, const uint64_t *key, int64_t np, TreeBuffers &tb, uint32_t *cube_start,
-                  cudaStream_t st, int64_t *launches) {
-  if (direct_applies(tp)) {
-    tree_units(tp, tb, st, launches);
-  } else {
-    const int cbits = kAxisBits - tp.sub_bits;
-    tree_groups(tp, key, np, tb, cube_start, 1ll << (3 * (cbits - tp.group_level)), 3 * (tp.sub_bits + tp.group_level),
-                st, launches);
-  }
+  k_write_groups<<<blocks, 256, 0, st>>>(start, ncubes, goff, bsum, tb.groups, gmax);
+  if (launches) *launches += 4;
 }
 
 // ------------------------------------------------------------------ walk
@@ -894,7 +878,6 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_tree_walk(
   float4 *tq = smem4 + kLogSmemF4;
   WarpLists *lists = reinterpret_cast<WarpLists *>(smem4 + kLogSmemF4 + kPcEntries + 1);
   const uint32_t ngroups = nbox == 1 ? boxes[0].counters[kCntGroups] : gprefix[nbox];
-  if (ngroups == 0) return;  // the direct summation took every cube
   for (int i = threadIdx.x; i <= kLogEntries; i += kWalkThreads) tl[i] = glog[i];
   for (int i = threadIdx.x; i <= kPcEntries; i += kWalkThreads) tq[i] = gpc[i];
   __syncthreads();
@@ -1235,7 +1218,6 @@ WalkBox walk_box(const TreeParams &tp, const uint32_t *spos, const TreeBuffers &
   b.mom1 = tb.mom1;
   b.mom2 = tb.mom2;
   b.groups = tb.groups;
-  b.units = tb.units;
   b.counters = tb.counters;
   b.ftree = ftree;
   b.err = err;
@@ -1268,34 +1250,25 @@ __global__ void k_set_walkbox(WalkBox *dst, WalkBox v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *dst = v;
 }
 
-void tree_direct(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb, const LawTable &law,
-                 float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches) {
-  // the box record goes to the device with the launch that precedes the sum
+void tree_walk(const TreeParams &tp, const uint32_t *spos, int64_t np, const TreeBuffers &tb,
+               const LawTable &law, float *ftree, uint32_t *err, cudaStream_t st, int64_t *launches) {
+  (void)np;
+  // the box record goes to the device with the launch that precedes the walk
   k_set_walkbox<<<1, 32, 0, st>>>(tb.walkbox, walk_box(tp, spos, tb, ftree, err));
-  if (launches) *launches += 1;
-  // the next-item counters were zeroed before tree_groups / tree_units
-  if (direct_applies(tp)) {
-    launch_direct(tb.walkbox, nullptr, 1, std::min(np, tb.ncubes4), &tb.counters[kCntNextUnit], tb.counters, law,
-                  tp.rsphere, st);
-    if (launches) *launches += 1;
-  }
-}
-
-void tree_walk(const TreeParams &tp, const TreeBuffers &tb, const LawTable &law, cudaStream_t st, int64_t *launches) {
+  // the next-group counter was zeroed before tree_groups
   launch_walk(tb.walkbox, nullptr, 1, &tb.counters[kCntNextGroup], tb.stack, tb.stack_words, tb.counters, law,
               tp.rsphere, st);
-  if (launches) *launches += 1;
+  if (launches) *launches += 2;
 }
 
-// Prefix of the boxes' group (or unit) counts, counters[word], and the
-// launch's next-item counter.
-__global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, int word, uint32_t *__restrict__ gprefix,
+// Prefix of the boxes' group counts and the launch's next-group counter.
+__global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, uint32_t *__restrict__ gprefix,
                                uint32_t *__restrict__ gnext) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     uint32_t run = 0;
     for (int b = 0; b < nbox; b++) {
       gprefix[b] = run;
-      run += boxes[b].counters[word];
+      run += boxes[b].counters[kCntGroups];
     }
     gprefix[nbox] = run;
     *gnext = 0;
@@ -1304,11 +1277,7 @@ __global__ void k_group_prefix(const WalkBox *__restrict__ boxes, int nbox, int 
 
 void tree_walk_multi(const WalkBox *boxes, int nbox, uint32_t *gprefix, uint32_t *gnext, uint32_t *stack,
                      int64_t stack_words, uint32_t *stats, const LawTable &law, float rsphere, cudaStream_t st) {
-  // every box's direct summation first: it leaves the groups of the cubes it
-  // cannot take in the boxes' group lists
-  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntUnits, gprefix, gnext);
-  launch_direct(boxes, gprefix, nbox, 1ll << 40, gnext, stats, law, rsphere, st);
-  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, kCntGroups, gprefix, gnext);
+  k_group_prefix<<<1, 32, 0, st>>>(boxes, nbox, gprefix, gnext);
   launch_walk(boxes, gprefix, nbox, gnext, stack, stack_words, stats, law, rsphere, st);
 }
 

@@ -67,9 +67,8 @@ TreeParams tree_params(const tpm_ctx *c) {
 void groups_and_walk(tpm_ctx *c) {
   TreeParams tp = tree_params(c);
   cudaMemsetAsync(c->tb.counters, 0, sizeof(uint32_t) * 16, c->st);
-  tree_targets(tp, c->skey, c->np, c->tb, c->cube_start, c->st, nullptr);
-  tree_direct(tp, c->spos, c->np, c->tb, c->law, c->ftree, c->err, c->st, nullptr);
-  tree_walk(tp, c->tb, c->law, c->st, nullptr);
+  tree_groups(tp, c->skey, c->np, c->tb, c->cube_start, c->st, nullptr);
+  tree_walk(tp, c->spos, c->np, c->tb, c->law, c->ftree, c->err, c->st, nullptr);
 }
 
 }  // namespace
@@ -103,8 +102,8 @@ int tpm_autotune(tpm_ctx *c, unsigned what, tpm_tuning *out) {
   if (!c) return fail(TPM_E_ARG, "ctx is NULL");
   if (c->np <= 0) return fail(TPM_E_STATE, "no particles loaded");
   CK(cudaSetDevice(c->device));
-  // one evaluation leaves sorted keys, the mesh and the whole tree in place
-  int rc = enqueue_forces(c, TPM_PART_ALL, c->st, false, true, true);
+  // one evaluation leaves sorted keys, the mesh and the tree in place
+  int rc = enqueue_forces(c, TPM_PART_ALL, c->st, false);
   if (!rc) rc = finish_forces(c, TPM_PART_ALL, false, false);
   if (rc) return rc;
   tpm_tuning res;
