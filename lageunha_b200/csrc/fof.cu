@@ -112,21 +112,21 @@ __global__ void __launch_bounds__(kFofThreads) k_fof_link(const uint32_t *__rest
       rest &= ~members;
       const bool mine = (members >> lane) & 1u;
       const uint32_t first = (uint32_t)(base + lead);
-      // the members' box, relative to the first of them
-      float mid[3], half[3], at[3];
-      uint32_t ref[3];
+      // the members' box: its middle (fixed point and cells) and half sizes
+      float half[3], at[3];
+      uint32_t mid[3];
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        ref[a] = __shfl_sync(0xffffffffu, p[a], lead);
-        float x = mine ? wrapf(p[a], ref[a], cpu) : 0.f, lo = x, hi = x;
+        const uint32_t ref = __shfl_sync(0xffffffffu, p[a], lead);
+        float x = mine ? wrapf(p[a], ref, cpu) : 0.f, lo = x, hi = x;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
           lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
           hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
         }
-        mid[a] = 0.5f * (lo + hi);
         half[a] = 0.5f * (hi - lo);
-        at[a] = __uint2float_rn(ref[a]) * cpu + mid[a];
+        at[a] = __uint2float_rn(ref) * cpu + 0.5f * (lo + hi);
+        mid[a] = ref + (uint32_t)__float2int_rn(0.5f * (lo + hi) / cpu);
       }
       // joins the members to the particles of [s, e) that are linked to them
       auto join = [&](uint32_t s, uint32_t e, bool clique, bool near) {
@@ -212,9 +212,11 @@ __global__ void __launch_bounds__(kFofThreads) k_fof_link(const uint32_t *__rest
           int kind = 0;  // 1: open, 2: join
           const uint32_t nch = rec.w & 0xffffu;
           if (has && rec.x + rec.y > first) {
-            float dx = fmaxf(fabsf(wrapf(geo.x, ref[0], cpu) - mid[0]) - nh - half[0], 0.f);
-            float dy = fmaxf(fabsf(wrapf(geo.y, ref[1], cpu) - mid[1]) - nh - half[1], 0.f);
-            float dz = fmaxf(fabsf(wrapf(geo.z, ref[2], cpu) - mid[2]) - nh - half[2], 0.f);
+            // the image nearest to the middle of the box has the smallest gap to
+            // it (the one nearest to a member at its edge may be on the far side)
+            float dx = fmaxf(fabsf(wrapf(geo.x, mid[0], cpu)) - nh - half[0], 0.f);
+            float dy = fmaxf(fabsf(wrapf(geo.y, mid[1], cpu)) - nh - half[1], 0.f);
+            float dz = fmaxf(fabsf(wrapf(geo.z, mid[2], cpu)) - nh - half[2], 0.f);
             // the box's own rounding beside the pair's
             if (dx * dx + dy * dy + dz * dz <= near2 + 1e-6f) kind = nch == 0 || (clique && rec.y <= 32u) ? 2 : 1;
           }

@@ -84,3 +84,21 @@ def test_fof_cubes_and_cliques(kind, n, link, minm):
         lab, ng = eng.fof(link, minm)
     assert ng == ngw
     assert np.array_equal(lab.astype(np.int64), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_fof_nodes_beyond_half_the_box_from_the_first_member(axis):
+    """The two members of one 4-cell cube lie 3.8 cells apart; the node of the
+    other ten is within the link of the second, and more than half the box from
+    the first."""
+    n, link = 16, 5.0
+    x = np.concatenate([[0.1, 3.9], np.linspace(8.5, 8.8, 10)])
+    pos = np.roll(np.stack([x, np.ones(12), np.ones(12)], 1), axis, axis=1)
+    pu = ic.to_fixed_point(pos, n)
+    want, ngw = O.fof_labels(n, ic.from_fixed_point(pu, n), link, 1)
+    assert ngw == 1
+    with E.Engine(n, epsilon=0.05) as eng:
+        eng.load_fixed(pu)
+        lab, ng = eng.fof(link, 1)
+    assert ng == ngw and np.array_equal(lab.astype(np.int64), want)
