@@ -20,10 +20,15 @@ using namespace tpm;
 
 namespace {
 
-// nodes a warp holds: while 32 opened nodes of eight children fit, 32 are taken
-// at a time, then one (which adds at most 7 on each of the 11 levels below a cube)
-constexpr int kFofStack = 768;
+// Nodes a warp holds. 32 are taken at a time while their children, eight each,
+// leave room for what single ones may still add: a node taken alone adds at most
+// 7 on each level below a cube, of which the smallest mesh (16 cells, 2 levels of
+// cubes) has most. So no set of particles can overflow it. 544 entries are the
+// most before a wide step.
+constexpr int kFofDeep = 7 * (kAxisBits - 2), kFofWide = 7 * 32;
+constexpr int kFofStack = 544 + kFofWide + kFofDeep;
 constexpr int kFofThreads = 128;
+static_assert(kFofStack * sizeof(uint32_t) * (kFofThreads / 32) * 16 <= 227 * 1024, "16 blocks per SM");
 
 TPM_D uint32_t find_root(uint32_t *parent, uint32_t x) {
   uint32_t p = parent[x];
@@ -196,8 +201,7 @@ __global__ void __launch_bounds__(kFofThreads) k_fof_link(const uint32_t *__rest
         int top = __popc(nodes);
         __syncwarp();
         while (top > 0) {
-          // fewer at a time when their children might not fit
-          const int take = min(top, top + 7 * 32 <= kFofStack ? 32 : 1);
+          const int take = min(top, top + kFofWide + kFofDeep <= kFofStack ? 32 : 1);
           const bool has = lane < take;
           uint4 rec = make_uint4(0, 0, 0, 0), geo = rec;
           if (has) {

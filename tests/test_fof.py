@@ -102,3 +102,42 @@ def test_fof_nodes_beyond_half_the_box_from_the_first_member(axis):
         eng.load_fixed(pu)
         lab, ng = eng.fof(link, 1)
     assert ng == ngw and np.array_equal(lab.astype(np.int64), want)
+
+
+def _stack_set():
+    """5955 particles, five in each of some cells of a nested subdivision of the
+    16-cell box, for which the search of the first warp (link 7.5: every 4-cell
+    cube is near) opens 32 nodes on three levels, then single ones down to 544
+    waiting nodes, then 32 more and one: 775 nodes wait, above the 768 that the
+    wide steps alone can reach."""
+    rng = np.random.Generator(np.random.PCG64(3))
+    out = []
+
+    def split(path):
+        c, *o = path
+        return (c >= 60, c == 63 and o[0] >= 4, c == 63 and o[0] == 5 and len(o) > 1 and o[1] < 4,
+                c == 63 and o[0] == 5 and o[1:] == [3, 7, 7], False)[len(o) - 1]
+
+    def cell(lo, side, path):
+        for o in range(8):
+            b = lo + side / 2 * np.array([o & 1, o >> 1 & 1, o >> 2])
+            if split(path + (o,)):
+                cell(b, side / 2, path + (o,))
+            else:
+                out.append(b + side / 2 * (0.1 + 0.8 * rng.random((5, 3))))
+
+    for c in range(64):
+        cell(4.0 * np.array([c % 4, c // 4 % 4, c // 16]), 4.0, (c,))
+    return np.concatenate(out)
+
+
+@pytest.mark.gpu
+def test_fof_search_holds_every_node():
+    n, link = 16, 7.5
+    pos = _stack_set()
+    assert len(pos) == 5955
+    with E.Engine(n, epsilon=0.05) as eng:
+        eng.load_fixed(ic.to_fixed_point(pos, n))
+        lab, ng = eng.fof(link, 2)
+    # neighbouring octants lie closer than the link: one group
+    assert ng == 1 and np.all(lab == 0)
