@@ -756,7 +756,7 @@ int tpm::enqueue_forces(tpm_ctx *c, unsigned parts, cudaStream_t st, bool timing
   // ---- sort
   if (sweep_sorts(np)) {
     c->perm = sweep_sort(c->pos, np, (uint32_t)g.n, g.sub_bits, reinterpret_cast<uint32_t *>(c->key_alt), c->val,
-                         c->val_alt, c->ss.hist, c->err, st, &c->launches);
+                         c->val_alt, c->ss.hist, st, &c->launches);
     c->skey = c->key;
   } else {
     launch_make_keys(c->pos, np, (uint32_t)g.n, g.sub_bits, c->key, c->val, st);
@@ -861,7 +861,6 @@ int tpm::finish_forces(tpm_ctx *c, unsigned parts, bool from_host, bool timing) 
     if (herr[0] & kErrNodeOverflow) return fail(TPM_E_OVERFLOW, "tree node capacity exceeded");
     if (herr[0] & kErrStackOverflow) return fail(TPM_E_OVERFLOW, "tree-walk stack overflow");
     if (herr[0] & kErrTmaTimeout) return fail(TPM_E_CUDA, "TMA load timed out in fda4");
-    if (herr[0] & kErrSortWait) return fail(TPM_E_CUDA, "a sort tile waited too long for its predecessor");
     return fail(TPM_E_CUDA, "device error flags 0x%x", herr[0]);
   }
   if (timing) {

@@ -16,7 +16,6 @@ enum DeviceError : uint32_t {
   kErrNodeOverflow = 2u,     // tree node capacity exceeded
   kErrTmaTimeout = 4u,       // a TMA transaction did not complete in time
   kErrListOverflow = 8u,     // interaction list overflow
-  kErrSortWait = 16u,        // a sort tile's predecessor did not report in time
 };
 
 // ---------------------------------------------------------------- sort
@@ -42,10 +41,10 @@ int64_t sort_tiles(int64_t np);
 bool sweep_sorts(int64_t np);
 int64_t sweep_words(int64_t np);
 uint32_t *sweep_sort(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits, uint32_t *key32, uint32_t *val,
-                     uint32_t *val_alt, uint32_t *scratch, uint32_t *err, cudaStream_t st, int64_t *launches);
+                     uint32_t *val_alt, uint32_t *scratch, cudaStream_t st, int64_t *launches);
 // Positions, full keys and cube ranges (launch_range_table's, of the keys >>
 // shift) of the sorted particles.
-void launch_gather_pos(const uint32_t *pos, uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
+void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
                        uint64_t *skey, int shift, uint32_t ntable, uint32_t *start, cudaStream_t st);
 // start[t] = first sorted index whose key >> shift >= t, t in [0, ntable].
 // (A Morton cube's eight sub-cubes are consecutive, so the table of the 4-cell

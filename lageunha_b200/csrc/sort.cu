@@ -18,6 +18,7 @@
 // and a scan per pass, 64-bit keys) remains for callers without scratch for
 // the look-back (tpm_morton_order_noalloc) and for 2^30 particles and more.
 #include "engine_internal.cuh"
+#include "lookback.h"
 
 namespace tpm {
 
@@ -266,9 +267,8 @@ constexpr int kLowBits = kKeyBits - 32;  // sorted by the first pass and dropped
 // words before the tile states: the digit counts of every pass and the passes'
 // tile tickets
 constexpr int kSweepHead = kSweepPasses * 256 + 8;
-// A tile's word per digit: its own count (kOwn) or that of all tiles up to and
-// with it (kAll)
-constexpr uint32_t kOwn = 1u << 30, kAll = 2u << 30, kCount = kOwn - 1u;
+// looks at its predecessors' words after which a tile counts their items itself
+constexpr uint32_t kSweepLooks = 1u << 22;
 
 int64_t sweep_words(int64_t np) { return kSweepHead + 256 * kSweepPasses * ((np + kSweepTile - 1) / kSweepTile); }
 
@@ -326,6 +326,23 @@ __global__ void __launch_bounds__(512) k_sweep_count(const uint32_t *__restrict_
   }
 }
 
+// The items of a full tile, from item i0 on, with digit d of the first pass and
+// of the others.
+__device__ __noinline__ uint32_t count_low_digit(const uint32_t *pos, int64_t i0, uint32_t n, int sub_bits, uint32_t d) {
+  uint32_t c = 0;
+  for (int64_t i = i0; i < i0 + kSweepTile; i++) {
+    uint32_t lo, hi;
+    key_halves(pos, i, n, sub_bits, lo, hi);
+    c += (lo & ((1u << kLowBits) - 1u)) == d ? 1u : 0u;
+  }
+  return c;
+}
+__device__ __noinline__ uint32_t count_digit(const uint32_t *key, int64_t i0, int shift, uint32_t d) {
+  uint32_t c = 0;
+  for (int64_t i = i0; i < i0 + kSweepTile; i++) c += ((key[i] >> shift) & 0xffu) == d ? 1u : 0u;
+  return c;
+}
+
 // One pass over one tile of kSweepTile items. kFirst: the items are the
 // particles in the caller's order, the digit the key's low bits; else (key,
 // index) pairs with the digit at `shift` of the 32-bit key. kLast: the keys are
@@ -337,13 +354,14 @@ __global__ void __launch_bounds__(512) k_sweep_count(const uint32_t *__restrict_
 // counter's updates runs at the shared memory's rate and not at its latency.
 // Tiles take their numbers in the order in which they start, so a tile's
 // predecessors are running or done when it looks back at them, and every wait
-// ends; it is bounded all the same (err gets kErrSortWait).
+// ends; should one be stalled all the same, its items are counted instead, so the
+// pass has one result.
 template <bool kFirst, bool kLast>
 __global__ void __launch_bounds__(kSweepThreads, 2)
     k_sweep_pass(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                  uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t np, uint32_t n, int sub_bits,
                  int shift, const uint32_t *__restrict__ counts, uint32_t *__restrict__ ticket,
-                 uint32_t *__restrict__ state, uint32_t *__restrict__ err) {
+                 uint32_t *__restrict__ state) {
   extern __shared__ __align__(16) uint32_t sw_smem[];
   uint32_t *sk = sw_smem, *sv = sk + kSweepTile;                          // the tile in digit order
   uint32_t(*wc)[256] = reinterpret_cast<uint32_t(*)[256]>(sv + kSweepTile);  // [warps][256]
@@ -438,29 +456,13 @@ __global__ void __launch_bounds__(kSweepThreads, 2)
       pg += wg[w];
     }
     lstart[tid] = px + x - run;
-    // look back, four tiles at a time
-    uint32_t before = 0;
-    int64_t t = tile - 1;
-    uint32_t spins = 0;
-    while (t >= 0) {
-      uint32_t s[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        s[q] = t - q >= 0 ? *reinterpret_cast<const volatile uint32_t *>(state + (t - q) * 256 + tid) : kAll;
-      bool done = false;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (done || s[q] < kOwn) break;
-        before += s[q] & kCount;
-        t--;
-        done = s[q] >= kAll;
-      }
-      if (done) break;
-      if (++spins > (1u << 22)) {
-        atomicOr(err, (uint32_t)kErrSortWait);
-        break;
-      }
-    }
+    const uint32_t before = items_before(
+        tile, kSweepLooks,
+        [&](int64_t t) { return *reinterpret_cast<const volatile uint32_t *>(state + t * 256 + tid); },
+        [&](int64_t t) {  // a tile with tiles after it is full
+          return kFirst ? count_low_digit(pos, t * kSweepTile, n, sub_bits, (uint32_t)tid)
+                        : count_digit(kin, t * kSweepTile, shift, (uint32_t)tid);
+        });
     if (tile > 0) *reinterpret_cast<volatile uint32_t *>(mine) = (before + run) | kAll;
     gbase[tid] = pg + g - total + before;
   }
@@ -498,7 +500,7 @@ constexpr size_t kSweepSmemFirst = kSweepSmem + kSweepTile;
 bool sweep_sorts(int64_t np) { return np < (int64_t)kOwn; }
 
 uint32_t *sweep_sort(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits, uint32_t *key32, uint32_t *val,
-                     uint32_t *val_alt, uint32_t *scratch, uint32_t *err, cudaStream_t st, int64_t *launches) {
+                     uint32_t *val_alt, uint32_t *scratch, cudaStream_t st, int64_t *launches) {
   const int64_t ntiles = (np + kSweepTile - 1) / kSweepTile;
   uint32_t *counts = scratch, *tickets = scratch + kSweepPasses * 256, *state = scratch + kSweepHead;
   uint32_t *ka = key32, *kb = key32 + np;
@@ -512,16 +514,16 @@ uint32_t *sweep_sort(const uint32_t *pos, int64_t np, uint32_t n, int sub_bits, 
   if (blocks > 148 * 4) blocks = 148 * 4;
   k_sweep_count<<<blocks, 512, 0, st>>>(pos, np, n, sub_bits, counts);
   k_sweep_pass<true, false><<<(unsigned)ntiles, kSweepThreads, kSweepSmemFirst, st>>>(
-      pos, nullptr, nullptr, ka, val, np, n, sub_bits, 0, counts, tickets, state, err);
+      pos, nullptr, nullptr, ka, val, np, n, sub_bits, 0, counts, tickets, state);
   uint32_t *vi = val, *vo = val_alt;
   for (int p = 1; p < kSweepPasses; p++) {
     uint32_t *stp = state + (int64_t)p * 256 * ntiles;
     if (p < kSweepPasses - 1)
       k_sweep_pass<false, false><<<(unsigned)ntiles, kSweepThreads, kSweepSmem, st>>>(
-          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp, err);
+          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp);
     else
       k_sweep_pass<false, true><<<(unsigned)ntiles, kSweepThreads, kSweepSmem, st>>>(
-          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp, err);
+          pos, ka, vi, kb, vo, np, n, sub_bits, 8 * (p - 1), counts + p * 256, tickets + p, stp);
     uint32_t *t = ka;
     ka = kb;
     kb = t;
@@ -554,7 +556,7 @@ TPM_D void range_entries(int64_t tp, int64_t t, int64_t i, uint32_t *__restrict_
 
 // The sorted particles: their positions, full keys and the range table of the
 // cubes key >> shift (ntable of them).
-__global__ void __launch_bounds__(256) k_gather_pos(const uint32_t *__restrict__ pos, uint32_t *__restrict__ perm,
+__global__ void __launch_bounds__(256) k_gather_pos(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ perm,
                                                     int64_t np, uint32_t n, int sub_bits, uint32_t *__restrict__ spos,
                                                     uint64_t *__restrict__ skey, int shift, uint32_t ntable,
                                                     uint32_t *__restrict__ start) {
@@ -565,7 +567,6 @@ __global__ void __launch_bounds__(256) k_gather_pos(const uint32_t *__restrict__
     uint64_t k = (uint64_t)ntable << shift;
     if (i < np) {
       int64_t p = perm[i];
-      if (p >= np) perm[i] = (uint32_t)(p = 0);  // only after a sort that gave up (kErrSortWait)
       const uint32_t u[3] = {pos[3 * p + 0], pos[3 * p + 1], pos[3 * p + 2]};
       k = key_of(u, 0, n, sub_bits);
       spos[3 * i + 0] = u[0];
@@ -575,13 +576,13 @@ __global__ void __launch_bounds__(256) k_gather_pos(const uint32_t *__restrict__
     }
     int64_t t = (int64_t)(k >> shift);
     int64_t tp = __shfl_up_sync(0xffffffffu, t, 1);
-    if (lane == 0) tp = i > 0 && i <= np ? (int64_t)(key_of(pos, min((int64_t)perm[i - 1], np - 1), n, sub_bits) >> shift) : -1;
+    if (lane == 0) tp = i > 0 && i <= np ? (int64_t)(key_of(pos, perm[i - 1], n, sub_bits) >> shift) : -1;
     if (i > np) t = tp;
     range_entries(tp, t, i, start);
   }
 }
 
-void launch_gather_pos(const uint32_t *pos, uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
+void launch_gather_pos(const uint32_t *pos, const uint32_t *perm, int64_t np, uint32_t n, int sub_bits, uint32_t *spos,
                        uint64_t *skey, int shift, uint32_t ntable, uint32_t *start, cudaStream_t st) {
   int blocks = (int)((np + 256) / 256);
   if (blocks > 148 * 32) blocks = 148 * 32;
