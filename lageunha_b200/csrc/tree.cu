@@ -877,7 +877,6 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_tree_walk(
   float2 *tl = reinterpret_cast<float2 *>(smem4);
   float4 *tq = smem4 + kLogSmemF4;
   WarpLists *lists = reinterpret_cast<WarpLists *>(smem4 + kLogSmemF4 + kPcEntries + 1);
-  const uint32_t ngroups = nbox == 1 ? boxes[0].counters[kCntGroups] : gprefix[nbox];
   for (int i = threadIdx.x; i <= kLogEntries; i += kWalkThreads) tl[i] = glog[i];
   for (int i = threadIdx.x; i <= kPcEntries; i += kWalkThreads) tq[i] = gpc[i];
   __syncthreads();
@@ -889,6 +888,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm) k_tree_walk(
   int max_top = 0;
   const uint32_t lanemask_lt = (1u << lane) - 1u;
   int cur_box = -1;
+  const uint32_t ngroups = nbox == 1 ? boxes[0].counters[kCntGroups] : gprefix[nbox];
   while (true) {
     uint32_t g = 0;
     if (lane == 0) g = atomicAdd(gnext, 1u);
