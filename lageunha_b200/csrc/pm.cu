@@ -1301,7 +1301,8 @@ TPM_D float3 fda_interp(const float *gx, const float *gy, const float *gz, uint3
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     // a plane's 27 loads are issued before the first is used: left to itself
-    // the compiler keeps few in flight
+    // the compiler keeps few in flight. They read what other threads wrote before
+    // the barrier, which the clobber tells the compiler.
     const float *const plane[3] = {gx + at + kGradSz * kStep[c], gy + at + kGradSz * kStep[c],
                                    gz + at + kGradSz * kStep[c]};
     float g[3][9];
@@ -1311,7 +1312,8 @@ TPM_D float3 fda_interp(const float *gx, const float *gy, const float *gz, uint3
       for (int e = 0; e < 3; e++)
         asm volatile("ld.shared.f32 %0, [%1];"
                      : "=f"(g[e][q])
-                     : "r"(smem_u32(plane[e] + kStep[q % 3] + kGradSy * kStep[q / 3])));
+                     : "r"(smem_u32(plane[e] + kStep[q % 3] + kGradSy * kStep[q / 3]))
+                     : "memory");
 #pragma unroll
     for (int q = 0; q < 9; q++) {
       float wt = wxs[q % 3] * wys[q / 3] * wzs[c];
