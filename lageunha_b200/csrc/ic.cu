@@ -29,6 +29,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "tpm_engine.h"
 #include "engine_internal.cuh"
 
@@ -603,25 +605,38 @@ int ic_fail(int code, const char *m) {
   return code;
 }
 
-// The device buffers of one call, carved from one allocation: a call makes up
-// to twenty-five of them, and a cudaMalloc and cudaFree for each took as long
-// as the kernels (4 ms at 256^3).
-struct Carve {
+// Buffers laid out one after another in one piece of memory.
+struct Layout {
   static constexpr int kMax = 32;
   void **at[kMax];
   size_t off[kMax], total = 0;
   int count = 0;
-  char *base = nullptr;
   template <class T>
   void add(T **p, size_t bytes) {
     at[count] = reinterpret_cast<void **>(p);
     off[count++] = total;
     total += (bytes + 255) / 256 * 256;
   }
+  void place(char *base) const {
+    for (int i = 0; i < count; i++) *at[i] = base + off[i];
+  }
+};
+
+// The device buffers of one call, carved from one allocation: a call makes up
+// to twenty-five of them, and a cudaMalloc and cudaFree for each took as long
+// as the kernels (4 ms at 256^3). The noise's scratch, read no more once the
+// spectrum is filled, lies over the meshes that are written after that.
+struct Carve : Layout {
+  char *base = nullptr;
+  Layout noise, meshes;
+  char *over = nullptr;  // both of them
   cudaError_t commit() {
+    add(&over, meshes.total > noise.total ? meshes.total : noise.total);
     cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), total);
     if (e != cudaSuccess) return e;
-    for (int i = 0; i < count; i++) *at[i] = base + off[i];
+    place(base);
+    noise.place(over);
+    meshes.place(over);
     return e;
   }
   ~Carve() { cudaFree(base); }
@@ -657,18 +672,18 @@ void noise_plan(const tpm_ic_params *p, Noise &w, Carve &mem) {
   w.nlev[0] = (trials + kTrialsPerChunk - 1) / kTrialsPerChunk;
   for (int l = 1; l < kLevels; l++) w.nlev[l] = (w.nlev[l - 1] + kRadix - 1) / kRadix;
   const int64_t nb = (w.nlev[0] + 4095) / 4096, rnb = (rows + 4095) / 4096;
-  mem.add(&w.x0, sizeof(uint32_t) * kLag);
-  mem.add(&w.jump, sizeof(uint32_t) * kLag * kLevels);
-  for (int l = 0; l < kLevels; l++) mem.add(&w.lev[l], sizeof(uint32_t) * kLag * w.nlev[l]);
-  mem.add(&w.counts, sizeof(uint32_t) * w.nlev[0]);
-  mem.add(&w.offs, sizeof(uint32_t) * w.nlev[0]);
-  mem.add(&w.bsum, sizeof(uint32_t) * (nb + 1));
-  mem.add(&w.total, sizeof(uint32_t) * 2);
-  mem.add(&w.rowcnt, sizeof(uint32_t) * rows);
-  mem.add(&w.rowoff, sizeof(uint32_t) * rows);
-  mem.add(&w.rbsum, sizeof(uint32_t) * (rnb + 1));
-  mem.add(&w.acc, sizeof(float2) * (w.modes > 0 ? w.modes : 1));
-  if (p->iseed < 0) mem.add(&w.velpot, sizeof(float) * (size_t)(knyq * knyq + 1));
+  mem.noise.add(&w.x0, sizeof(uint32_t) * kLag);
+  mem.noise.add(&w.jump, sizeof(uint32_t) * kLag * kLevels);
+  for (int l = 0; l < kLevels; l++) mem.noise.add(&w.lev[l], sizeof(uint32_t) * kLag * w.nlev[l]);
+  mem.noise.add(&w.counts, sizeof(uint32_t) * w.nlev[0]);
+  mem.noise.add(&w.offs, sizeof(uint32_t) * w.nlev[0]);
+  mem.noise.add(&w.bsum, sizeof(uint32_t) * (nb + 1));
+  mem.add(&w.total, sizeof(uint32_t) * 2);  // read at the end
+  mem.noise.add(&w.rowcnt, sizeof(uint32_t) * rows);
+  mem.noise.add(&w.rowoff, sizeof(uint32_t) * rows);
+  mem.noise.add(&w.rbsum, sizeof(uint32_t) * (rnb + 1));
+  mem.noise.add(&w.acc, sizeof(float2) * (w.modes > 0 ? w.modes : 1));
+  if (p->iseed < 0) mem.noise.add(&w.velpot, sizeof(float) * (size_t)(knyq * knyq + 1));
 }
 
 int row_grid(int n) { return n * n < 148 * 16 ? n * n : 148 * 16; }
@@ -777,7 +792,7 @@ int tpm_ic_zeldovich(const tpm_ic_params *p, void *records, int mem) {
   double rincube = 1. / (double)n / (double)n / (double)n;
   cudaStream_t st = nullptr;
   FftPlan plan;
-  float2 *phik = nullptr, *work = nullptr, *tw = nullptr;
+  float2 *phik = nullptr, *work = nullptr, *tw = nullptr, *spec = nullptr;
   float *pad[3] = {nullptr, nullptr, nullptr}, *real = nullptr;
   double *sums = nullptr;
   DmRecord *rec = reinterpret_cast<DmRecord *>(records);
@@ -788,8 +803,7 @@ int tpm_ic_zeldovich(const tpm_ic_params *p, void *records, int mem) {
     return ic_fail(TPM_E_CUDA, "cudaStreamCreate failed");
   noise_plan(p, noise, buf);
   buf.add(&phik, sizeof(float2) * elems);
-  buf.add(&work, sizeof(float2) * elems);
-  for (int a = 0; a < 3; a++) buf.add(&pad[a], pad_bytes);
+  for (int a = 0; a < 3; a++) buf.meshes.add(&pad[a], a < 2 ? pad_bytes : std::max(pad_bytes, sizeof(float2) * elems));
   buf.add(&sums, sizeof(double) * 2);
   buf.add(&tw, sizeof(float2) * fft_twiddles(n));
   if (mem != TPM_MEM_DEVICE) buf.add(&rec, sizeof(DmRecord) * cells);
@@ -802,14 +816,17 @@ int tpm_ic_zeldovich(const tpm_ic_params *p, void *records, int mem) {
   // conjugate completion (PMSeedForce.c:355-396) leaves the ky = n/2 and
   // kz = n/2 lines as drawn
   real = pad[1];  // free until the displacements
+  work = reinterpret_cast<float2 *>(pad[2]);  // free until the last of them
   IC_CK(cudaMemsetAsync(sums, 0, sizeof(double) * 2, st));
   fft_inverse(g, plan, phik, pad[0], st);
   k_phi_moments<<<row_grid(n), 128, 0, st>>>(pad[0], g, rincube, sums);
   k_phi_nongauss<<<row_grid(n), 128, 0, st>>>(pad[0], g, rincube, sums, p->fnl, p->gnl, real);
   fft_forward(g, plan, real, phik, st);
   for (int a = 0; a < 3; a++) {
-    k_psi_spec<<<row_grid(n), 128, 0, st>>>(n, g.hx, phik, a, work);
-    fft_inverse(g, plan, work, pad[a], st);
+    // the last component takes phi_k's place, whose memory it may overwrite
+    spec = a < 2 ? work : phik;
+    k_psi_spec<<<row_grid(n), 128, 0, st>>>(n, g.hx, phik, a, spec);
+    fft_inverse(g, plan, spec, pad[a], st);
   }
   k_records<<<row_grid(n), 128, 0, st>>>(pad[0], pad[1], pad[2], g, rincube, p->vamp, p->pfact, rec);
   IC_CK(cudaGetLastError());
@@ -858,7 +875,7 @@ int tpm_ic_2lpt(const tpm_ic_params *p, void *records, int mem) {
   buf.add(&s1, sizeof(float2) * elems);
   buf.add(&s2, sizeof(float2) * elems);
   buf.add(&work, sizeof(float2) * elems);
-  for (int a = 0; a < 3; a++) buf.add(&pad[a], pad_bytes);
+  for (int a = 0; a < 3; a++) buf.meshes.add(&pad[a], pad_bytes);
   buf.add(&sums, sizeof(double) * 2);
   buf.add(&tw, sizeof(float2) * fft_twiddles(n));
   if (mem != TPM_MEM_DEVICE) buf.add(&rec, sizeof(DmRecord) * cells);

@@ -299,3 +299,48 @@ def test_2lpt_non_gaussian_needs_the_cosmology():
     p.n, p.iseed, p.fnl = 16, 3, 10.0
     rec = np.empty(16 ** 3, E.DM_DTYPE)
     assert E.load_library().tpm_ic_2lpt(p, rec.ctypes.data, E.MEM_HOST) == -1  # TPM_E_ARG
+
+
+def _peak_bytes(call):
+    """The device memory that a call takes at most, sampled while it runs."""
+    import threading
+
+    import torch
+    torch.cuda.synchronize()
+    call()  # contexts and modules are loaded
+    free0 = torch.cuda.mem_get_info()[0]
+    low, stop = [free0], threading.Event()
+
+    def watch():
+        while not stop.is_set():
+            low[0] = min(low[0], torch.cuda.mem_get_info()[0])
+
+    t = threading.Thread(target=watch)
+    t.start()
+    try:
+        for _ in range(5):
+            call()
+    finally:
+        stop.set()
+        t.join()
+    return free0 - low[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2])
+def test_device_memory_of_a_call(order):
+    """A call with device records holds at most the arrays it works on at one
+    time: first order four of the mesh (spectra of n^2 (n / 2 + 1) complex numbers
+    or meshes with 8 ghost layers), second order six. The noise's scratch shares
+    their memory, and 24 MB are left for tables and the driver's granularity."""
+    import torch
+    n = 384
+    rec = torch.empty((n ** 3, 8), dtype=torch.float32, device="cuda")
+    vp = power_law_velpot(n)
+    if order == 1:
+        peak = _peak_bytes(lambda: E.ic_zeldovich(n, -5, vp, vamp=0.01, pfact=1.0, out=rec))
+    else:
+        peak = _peak_bytes(lambda: E.ic_2lpt(n, -5, vp, vamp=0.01, vamp2=-0.004, damp1=1.0, damp2=-0.4, pfact=1.0 / n, out=rec))
+    mesh, spec = 4 * (n + 16) ** 3, 8 * n * n * (n // 2 + 1)
+    assert peak > 3 * spec  # the samples caught the call
+    assert peak <= 3 * mesh + (1 if order == 1 else 3) * spec + (24 << 20)
