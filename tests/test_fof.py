@@ -57,12 +57,14 @@ def test_fof_singletons_and_no_groups():
 
 def _set(kind, n):
     """Positions for the cube search: clumps on the periodic corner and on
-    cube faces, dense enough for whole nodes to lie within the link, or a
-    sparse set with links across several cubes."""
+    cube faces, dense enough for whole nodes to lie within the link, a core
+    with short links, or a sparse set with links across several cubes."""
     rng = np.random.Generator(np.random.PCG64(77 + n))
     if kind == "clumps":
         c = np.array([[0, 0, 0], [4, 8, 4], [n - 1, 4, 0.02]], np.float64)
         p = np.concatenate([c[i % 3] + 0.08 * rng.standard_normal((400, 3)) for i in range(3)] + [rng.random((300, 3)) * n])
+    elif kind == "core":  # dense enough for a warp's particles to be split by octants
+        p = np.array([[8.0, 4.0, 0.0]]) + 0.3 * rng.standard_normal((2500, 3))
     else:
         p = rng.random((500, 3)) * n
     return ic.to_fixed_point(np.mod(p, n), n)
@@ -70,7 +72,8 @@ def _set(kind, n):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind,n,link,minm", [("clumps", 16, 0.2, 5), ("clumps", 45, 0.15, 2), ("clumps", 512, 0.25, 3),
-                                              ("sparse", 45, 3.0, 2), ("sparse", 16, 1.2, 1), ("sparse", 18, 5.0, 2)])
+                                              ("sparse", 45, 3.0, 2), ("sparse", 16, 1.2, 1), ("sparse", 18, 5.0, 2), ("core", 16, 0.02, 2),
+                                              ("core", 45, 0.06, 2), ("core", 512, 0.004, 2)])
 def test_fof_cubes_and_cliques(kind, n, link, minm):
     pu = _set(kind, n)
     pos = ic.from_fixed_point(pu, n)
