@@ -76,18 +76,21 @@ def test_groups_and_nodes_of_the_long_tiles(count):
     assert ng == ngw and np.array_equal(lab.astype(np.int64), want)
 
 
-@pytest.mark.parametrize("centre", [[18.0, 18.0, 18.0], [0.9, 31.2, 14.6]])
-def test_moments_of_an_accepted_node(centre):
-    """A lopsided clump of 400 particles in one 4-cell cube, and single ones
+@pytest.mark.parametrize("centre,scale", [([18.0, 18.0, 18.0], 1.0), ([0.9, 31.2, 14.6], 1.0),
+                                          ([18 + 0.5 / 256, 18 + 1.5 / 256, 18 + 2.5 / 256], 1.5e-3)])
+def test_moments_of_an_accepted_node(centre, scale):
+    """A lopsided clump of 400 particles in one 4-cell cube, or shrunk into one
+    cube of the deepest level (a leaf that a warp sums), and single ones
     around it that accept the cube's node as a whole (opening angle 0.9). Their
     force is the node's, with the clump's mass, centre and second moments, and
     the other single ones', all in FP64. The tolerance is four times the law
     tables' 2.8e-5 of the clump's Newtonian force, of which the terms of the
-    second moments are 0.2-2.5% and those beyond them up to 0.07%."""
+    second moments of the wide clump are 0.2-2.5% and those beyond up to 0.07%."""
     n, rs, eps = 32, np.float32(2.0).item(), np.float32(0.05).item()
     rng = np.random.Generator(np.random.PCG64(9))
     c = np.array(centre)
-    clump = c + np.clip(rng.standard_normal((400, 3)), -2.4, 2.4) * [0.34, 0.2, 0.1] + 0.25 * (rng.random((400, 1)) < 0.3)
+    clump = np.clip(rng.standard_normal((400, 3)), -2.4, 2.4) * [0.34, 0.2, 0.1] + 0.25 * (rng.random((400, 1)) < 0.3)
+    clump = c + scale * clump
     d = rng.standard_normal((4000, 3))
     around = d / np.linalg.norm(d, axis=1)[:, None] * (3.2 + 1.4 * rng.random((4000, 1)))
     around = around[np.abs(around).max(1) > 2.9]
@@ -105,6 +108,7 @@ def test_moments_of_an_accepted_node(centre):
         eng.compute(E.PART_TREE)
         f = eng.forces()[400:].astype(np.float64)
     assert len(around) >= 8 and len(np.unique(np.floor(np.mod(clump, n) / 4), axis=0)) == 1
+    assert scale == 1.0 or len(np.unique(O.morton_keys(pu[:400], n))) == 1
 
     from scipy.special import erf
 
